@@ -127,7 +127,15 @@ int chol_adjoint_one(mo_ctx *ctx, View L, View G, const AdjScratch &w, bool stre
     const View Dinv{w.Di, jb, jb, NBA};
     if (below > 0) {
       const View B = L.sub(j0 + jb, j0, below, jb), Bbar = G.sub(j0 + jb, j0, below, jb);
-      if ((rc = gemm_ex(ctx, Bbar, Bbar, false, Dinv, false, 1.0, 0.0, plain))) return rc;
+      // Bbar D^-1 in place, 128 columns at a time from the left (D^-1 is lower triangular, so
+      // a column block needs itself and the ones right of it): the engine's in-place tiles
+      // cover at most 128 columns
+      for (int c0 = 0; c0 < jb; c0 += NBI) {
+        const int cb = std::min(NBI, jb - c0);
+        if ((rc = gemm_ex(ctx, Bbar.sub(0, c0, below, cb), Bbar.sub(0, c0, below, jb - c0), false,
+                          Dinv.sub(c0, c0, jb - c0, cb), false, 1.0, 0.0, plain)))
+          return rc;
+      }
       // one 128 x 128 tile with K = rows below: as a plain product it is spread over the
       // device by stream-K (a triangle-mode launch would run on one SM); the strict upper
       // part of Dbar it also writes is never read and is overwritten at the end

@@ -148,8 +148,8 @@ int mo_ctx_create(int device, mo_ctx **out) {
   cudaError_t e = cudaMalloc(&ctx->d_status, sizeof(mo::Control));
   if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(mo::Control));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->sk_partial, mo::gemm_partial_bytes(ctx->sms));
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->sk_flags, sizeof(int) * ctx->sms);
-  if (e == cudaSuccess) e = cudaMemset(ctx->sk_flags, 0, sizeof(int) * ctx->sms);
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->sk_flags, 2 * sizeof(int) * ctx->sms);
+  if (e == cudaSuccess) e = cudaMemset(ctx->sk_flags, 0, 2 * sizeof(int) * ctx->sms);
   if (e != cudaSuccess) {
     if (ctx->sk_partial) cudaFree(ctx->sk_partial);
     if (ctx->sk_flags) cudaFree(ctx->sk_flags);

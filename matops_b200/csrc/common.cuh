@@ -78,10 +78,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, uint64_
 }
 
 // 8-byte cp.async with zero fill when src_bytes == 0
-__device__ __forceinline__ void cp_async_8(void *dst, const void *src, uint32_t src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+__device__ __forceinline__ void cp_async_8(uint32_t dst, const void *src, uint32_t src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src),
                "r"(src_bytes)
                : "memory");
+}
+__device__ __forceinline__ void cp_async_8(void *dst, const void *src, uint32_t src_bytes) {
+  cp_async_8(smem_u32(dst), src, src_bytes);
 }
 
 __device__ __forceinline__ void cp_async_arrive_noinc(uint64_t *bar) {

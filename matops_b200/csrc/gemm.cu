@@ -1,14 +1,28 @@
 // FP64 GEMM / SYRK engine for sm_100a.
 //
-// One CTA computes a 128x128 tile of C.  A producer warp streams 128x16 slabs of op(A)
-// and op(B) into a 6-stage shared-memory ring with 2-D TMA loads (128-byte swizzle, OOB
-// zero fill); eight consumer warps (2 x 4, 64 x 32 each) run the FP64 tensor pipe through
-// mma.sync.m16n8k4.f64 and hand stages back through mbarriers.  Operands whose base or
-// leading dimension breaks TMA's 16-byte rules (arbitrary FloatMatrix views) use the
-// same kernel with an 8-byte cp.async producer writing the identical swizzled layout.
-// A C at most 64 columns wide and at least 2048 rows tall (the FP64 residual of a solve
-// with few right-hand sides) takes 256x64 tiles in a 5-stage ring instead, with the
-// consumer warps arranged 4 x 2, so that none of them idles on columns past N.
+// A unit of work is one 128x64 tile of C, computed by one consumer warpgroup (2 x 2 warps
+// of 64 x 32) on the FP64 tensor pipe through mma.sync.m16n8k4.f64.  A CTA (one per SM)
+// runs two such warpgroups, each with its own list of units and its own 4-stage
+// shared-memory ring of 16-wide k-slabs of op(A) and op(B), filled by 2-D TMA (128-byte
+// swizzle, OOB zero fill) or, where the base or leading dimension breaks TMA's 16-byte
+// rules (arbitrary FloatMatrix views, e.g. an odd order), by 8-byte cp.async from two
+// producer warps per ring into the identical swizzled layout.
+//
+// Two independent warpgroups, because an epilogue (C read, scaled, written) leaves the
+// FP64 pipe idle: while one warpgroup writes its tile the other keeps multiplying.  A lone
+// warp per scheduler reaches about 0.85 of the pipe's rate, two reach 0.98, so both
+// multiply at once most of the time, the second one started half a tile late so that their
+// epilogues do not coincide.
+//
+// What bounds it: the FP64 pipe (37.0 TFLOP/s measured), plus per tile the C traffic, which
+// at K = 128 is a third of the tile's time.  Measured on B200, C -= A B, against one 128x128
+// tile per CTA shared by both warpgroups with a per-element epilogue: 8192^2 x K = 128 24.0 ->
+// 29.3 TFLOP/s, K = 256 28.6 -> 32.0; 16384^2 x 256 29.1 -> 32.7; 2048^3 33.2 -> 33.7;
+// 3001 x 1777 x 2503 with odd leading dimensions, op(A) = A^T, 12.8 -> 30.9 (one producer
+// warp before).
+//
+// Tiles are 64x128 (warps 1 x 4) where C is op(A) itself (in-place products from the right:
+// a tile must cover all its columns) or has at most 64 rows.
 //
 // Arithmetic (calgo/dmmat_gemm.c:364-415 semantics): C = beta*C + alpha*sum_k, with
 // beta == 0 never reading C.  SYRK modes restrict tiles and elements to one triangle and
@@ -28,27 +42,25 @@
 namespace mo {
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, STAGES = 6;
-constexpr int CONSUMER_WARPS = 8;
-// warpgroup 0 = producer (warp 0 issues the loads), warpgroups 1-2 = consumers.
+constexpr int BK = 16, STAGES = 4;  // stages per warpgroup
+constexpr int GROUP_WARPS = 4;  // warps of one consumer warpgroup
+// warpgroup 0 = producers (one warp per ring issues TMA loads, or two its cp.async copies),
+// warpgroups 1-2 = consumers.
 // Register split via setmaxnreg: launch 384 x 168 = 64512 = 128 x 40 + 256 x 232.
 constexpr int THREADS = 384;
 constexpr int PRODUCER_REGS = 40, CONSUMER_REGS = 232;
 static_assert(THREADS * 168 >= 128 * PRODUCER_REGS + 256 * CONSUMER_REGS, "register split");
-// Tile geometry of one instantiation.  NARROW (C at most 64 columns wide, e.g. a residual
-// B - A X with few right-hand sides): 256 x 64 tiles, warps in a 4 x 2 grid of the same
-// 64 x 32 warp tiles, so all eight consumer warps issue MMAs where a 128 x 128 tile would
-// leave half of them idle.
-template <bool NARROW>
+// Tile geometry of one instantiation: TALL 128 x 64, WIDE 64 x 128; warp tiles of 64 x 32.
+template <bool WIDE>
 struct Geo {
-  static constexpr int TBM = NARROW ? 256 : 128, TBN = NARROW ? 64 : 128;
-  static constexpr int NSTAGES = NARROW ? 5 : STAGES;
-  static constexpr int A_DBL = TBM * BK, B_DBL = TBN * BK, STAGE_DBL = A_DBL + B_DBL;
-  static constexpr uint32_t SBYTES = STAGE_DBL * 8;
-  static constexpr int SMEM = NSTAGES * SBYTES + 1024 + 2 * NSTAGES * 8;
-  static constexpr int WN = TBN / 32;  // warp columns
+  static constexpr int TBM = WIDE ? 64 : 128, TBN = WIDE ? 128 : 64;
+  static constexpr int WN = TBN / 32;  // warp columns of a warpgroup
 };
-static_assert(Geo<true>::SMEM <= 227 * 1024 && Geo<false>::SMEM <= 227 * 1024, "shared memory");
+constexpr int STAGE_DBL = (128 + 64) * BK;
+constexpr uint32_t STAGE_BYTES = STAGE_DBL * 8;
+constexpr int SMEM_BYTES = 2 * STAGES * STAGE_BYTES + 1024 + (4 * STAGES + 1) * 8;
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+constexpr int TILE_DBL = 128 * 64;  // elements of a tile (a stream-K partial)
 
 // Swizzled shared-memory layouts (TMA SWIZZLE_128B: 16-byte chunk ^= 128-byte row % 8).
 // K-major slab: 128 rows (m or n) of 16 k-values (128 B per row).
@@ -75,40 +87,54 @@ struct KParams {
   int tiles_m, tiles_n;
   int total_tiles;  // tiles of C (the triangle's tiles in SYRK modes)
   int kt;           // k-slabs per tile
-  int dp_tiles;     // tiles [0, dp_tiles) are processed whole, round-robin over CTAs
+  int workers;      // warpgroups with work of their own: 2 per CTA
+  int dp_tiles;     // tiles [0, dp_tiles) are processed whole, round-robin over workers
   int sk_iters;     // stream-K iterations over the remaining tiles
-  int sk_chunk;     // stream-K iterations per CTA
-  double *partial;  // [gridDim.x][64 * 256] stream-K partial accumulators
-  int *flags;       // [gridDim.x] epoch stamps of published partials
+  int sk_chunk;     // stream-K iterations per worker
+  double *partial;  // [workers][TILE_DBL] stream-K partial accumulators
+  int *flags;       // [workers] epoch stamps of published partials
   int epoch;
 };
 
 // cp.async producer for one ROWS x 16 slab (ROWS = 64 or 128) of an operand whose element
 // (mn, k) lives at src[k + mn*ld] (KMAJ) or src[mn + k*ld] (!KMAJ); out-of-range elements
-// are zero-filled.
-template <bool KMAJ, int ROWS = 128>
+// are zero-filled.  The two producer warps take half of the slab each (pw = 0, 1).
+template <bool KMAJ, int ROWS>
 __device__ __forceinline__ void load_slab_cpasync(double *dst, const double *src, int64_t ld,
-                                                  int mn0, int k0, int MN, int K, int lane) {
+                                                  int mn0, int k0, int MN, int K, int pw,
+                                                  int lane) {
   if constexpr (KMAJ) {
-#pragma unroll 8
-    for (int i = 0; i < ROWS / 2; ++i) {
-      int mn = 2 * i + (lane >> 4), k = lane & 15;
-      int gm = mn0 + mn, gk = k0 + k;
-      bool ok = gm < MN && gk < K;
-      const double *s = ok ? src + gk + (int64_t)gm * ld : src;
-      cp_async_8(dst + kmaj_off(mn, k), s, ok ? 8u : 0u);
+    // 16 lanes along k, two rows per instruction; 8 rows later the swizzle repeats
+    const int k = lane & 15, mn1 = (ROWS / 2) * pw + (lane >> 4);
+    const double *s = src + (k0 + k) + (int64_t)(mn0 + mn1) * ld;
+    const int left = k0 + k < K ? MN - mn0 - mn1 : 0;  // rows of this lane's column in range
+    uint32_t d[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) d[j] = smem_u32(dst + kmaj_off(mn1 + 2 * j, k));
+    const int64_t ld2 = 2 * ld;
+#pragma unroll 1
+    for (int i = 0; i < ROWS / 4; i += 4) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool ok = 2 * (i + j) < left;
+        cp_async_8(d[j] + i * (2 * 16 * 8), ok ? s : src, ok ? 8u : 0u);
+        s += ld2;
+      }
     }
   } else {
-#pragma unroll 4
-    for (int k = 0; k < 16; ++k)
+    const int left = MN - mn0 - lane;
+    const double *s = src + (mn0 + lane) + (int64_t)(k0 + 8 * pw) * ld;
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i) {
+      const int k = 8 * pw + i;
+      const int lim = k0 + k < K ? left : 0;
 #pragma unroll
       for (int j = 0; j < ROWS / 32; ++j) {
-        int mn = 32 * j + lane;
-        int gm = mn0 + mn, gk = k0 + k;
-        bool ok = gm < MN && gk < K;
-        const double *s = ok ? src + gm + (int64_t)gk * ld : src;
-        cp_async_8(dst + mnmaj_off(mn, k), s, ok ? 8u : 0u);
+        const bool ok = 32 * j < lim;
+        cp_async_8(smem_u32(dst + mnmaj_off(32 * j + lane, k)), ok ? s + 32 * j : src, ok ? 8u : 0u);
       }
+      s += ld;
+    }
   }
 }
 
@@ -125,47 +151,56 @@ __device__ __forceinline__ void tile_coords(const KParams &p, int t, int &tm, in
     tn = r / gm;
     return;
   }
-  // t enumerates the triangle row by row: (r, c) with c <= r
+  // t / 2 enumerates the triangle of 128 x 128 squares row by row, (r, c) with c <= r, and
+  // t & 1 the square's two tiles (the second one of a diagonal square may lie past N)
+  const int half = t & 1;
+  t >>= 1;
   int r = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
   while ((r + 1) * (r + 2) / 2 <= t) ++r;
   while (r * (r + 1) / 2 > t) --r;
   const int c = t - r * (r + 1) / 2;
   if (p.mode == kSyrkLower) {
     tm = r;
-    tn = c;
+    tn = 2 * c + half;
   } else {
     tm = c;
-    tn = r;
+    tn = 2 * r + half;
   }
 }
 
-// One unit of work: k-slabs [k0, k1) of tile `tile`.  owner: this CTA finishes the tile
-// (adds the partials of CTAs [first_contrib, blockIdx.x) and writes C); otherwise it
-// publishes its partial sum.
+// The worker index of a CTA's warpgroup: the first gridDim.x workers are the CTAs'
+// warpgroups 0, so that every SM has one before any has two.
+__device__ __forceinline__ int worker_of(const KParams &p, int grp) {
+  return grp * gridDim.x + blockIdx.x;
+}
+
+// One unit of work: k-slabs [k0, k1) of tile `tile`.  owner: this worker finishes the tile
+// (adds the partials of workers [first_contrib, w) and writes C); otherwise it publishes
+// its partial sum.
 struct Unit {
   int tile, k0, k1;
   bool owner;
   int first_contrib;
 };
 
-// Enumerates this CTA's units in processing order: whole tiles first, then its stream-K
-// range from the highest tile down (so that a partial is published before this CTA waits
-// for the partials of lower-numbered CTAs).  Returns the number of units; fills u[i] for
-// i == idx.
-__device__ __forceinline__ bool unit_at(const KParams &p, int idx, Unit &u) {
-  const int P = gridDim.x, b = blockIdx.x;
-  const int ndp = (p.dp_tiles > b) ? (p.dp_tiles - b + P - 1) / P : 0;
+// Worker w's units in processing order: whole tiles first, then its stream-K range from the
+// highest tile down (so that a partial is published before this worker waits for the
+// partials of lower-numbered ones).  Returns false past the last unit; fills u otherwise.
+__device__ __forceinline__ bool unit_at(const KParams &p, int w, int idx, Unit &u) {
+  const int P = p.workers;
+  if (w >= P) return false;
+  const int ndp = (p.dp_tiles > w) ? (p.dp_tiles - w + P - 1) / P : 0;
   if (idx < ndp) {
-    u.tile = b + idx * P;
+    u.tile = w + idx * P;
     u.k0 = 0;
     u.k1 = p.kt;
     u.owner = true;
-    u.first_contrib = b;
+    u.first_contrib = w;
     return true;
   }
   idx -= ndp;
   if (p.sk_iters <= 0) return false;
-  const int s = b * p.sk_chunk, e = min(s + p.sk_chunk, p.sk_iters);
+  const int s = w * p.sk_chunk, e = min(s + p.sk_chunk, p.sk_iters);
   if (s >= e) return false;
   const int first = s / p.kt, last = (e - 1) / p.kt;
   const int t = last - idx;
@@ -179,31 +214,32 @@ __device__ __forceinline__ bool unit_at(const KParams &p, int idx, Unit &u) {
   return true;
 }
 
-__device__ __forceinline__ void consumer_bar() {
-  asm volatile("bar.sync 1, 256;" ::: "memory");
+__device__ __forceinline__ void group_bar(int g) {
+  if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else asm volatile("bar.sync 2, 128;" ::: "memory");
 }
 
-template <bool A_KMAJ, bool B_KMAJ, bool USE_TMA, bool NARROW>
+template <bool A_KMAJ, bool B_KMAJ, bool USE_TMA, bool WIDE>
 __global__ void __launch_bounds__(THREADS, 1)
     dgemm_tile_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, const KParams p) {
-  using G = Geo<NARROW>;
-  constexpr int STAGES = G::NSTAGES;
+  using G = Geo<WIDE>;
   extern __shared__ unsigned char smem_raw[];
   const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023);
-  double *tiles = reinterpret_cast<double *>(base);
-  uint64_t *full = reinterpret_cast<uint64_t *>(base + STAGES * G::SBYTES);
-  uint64_t *empty = full + STAGES;
-  __shared__ int s_abort;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(base + 2 * STAGES * STAGE_BYTES);
+  uint64_t *late = bars + 4 * STAGES;  // warpgroup 0 is halfway through its first unit
+  __shared__ int s_abort[2];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (p.skip && *(volatile const int *)p.skip) return;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], USE_TMA ? 1u : 32u);
-      mbar_init(&empty[s], CONSUMER_WARPS);
-    }
-    s_abort = 0;
+    for (int r = 0; r < 2; ++r)
+      for (int s = 0; s < STAGES; ++s) {
+        mbar_init(&bars[2 * STAGES * r + s], USE_TMA ? 1u : 64u);             // full
+        mbar_init(&bars[2 * STAGES * r + STAGES + s], GROUP_WARPS);           // empty
+      }
+    mbar_init(late, GROUP_WARPS);
+    s_abort[0] = s_abort[1] = 0;
     fence_barrier_init();
   }
   __syncthreads();
@@ -211,10 +247,14 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp < 4) {
     // ------------------------------ producer warpgroup ------------------------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
-    if (warp != 0) return;
+    const int grp = USE_TMA ? warp : warp >> 1;  // ring
+    if (grp > 1) return;
+    uint64_t *full = bars + 2 * STAGES * grp, *empty = full + STAGES;
+    double *tiles = reinterpret_cast<double *>(base) + grp * STAGES * STAGE_DBL;
+    const int w = worker_of(p, grp);
     int it = 0;  // ring position, continues across units
     Unit u;
-    for (int ui = 0; unit_at(p, ui, u); ++ui) {
+    for (int ui = 0; unit_at(p, w, ui, u); ++ui) {
       int tm, tn;
       tile_coords(p, u.tile, tm, tn);
       const int m0 = tm * G::TBM, n0 = tn * G::TBN;
@@ -225,18 +265,15 @@ __global__ void __launch_bounds__(THREADS, 1)
           if constexpr (!USE_TMA) asm volatile("cp.async.wait_all;" ::: "memory");
           return;
         }
-        double *As = tiles + s * G::STAGE_DBL;
-        double *Bs = As + G::A_DBL;
+        double *As = tiles + s * STAGE_DBL;
+        double *Bs = As + G::TBM * BK;
         const int k0 = kt * BK;
         if constexpr (USE_TMA) {
           if (lane == 0) {
-            mbar_arrive_expect_tx(&full[s], G::SBYTES);
-            // K-major maps carry 128-row boxes (64 rows for a narrow B), MN-major maps
-            // 16 x 16 boxes
+            mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
+            // K-major maps carry boxes of the tile's rows, MN-major maps 16 x 16 boxes
             if (A_KMAJ) {
-#pragma unroll
-              for (int h = 0; h < G::TBM / 128; ++h)
-                tma_load_2d(As + h * 128 * BK, &tmA, &full[s], k0, m0 + 128 * h);
+              tma_load_2d(As, &tmA, &full[s], k0, m0);
             } else {
 #pragma unroll
               for (int bb = 0; bb < G::TBM / 16; ++bb)
@@ -252,11 +289,8 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           __syncwarp();
         } else {
-#pragma unroll
-          for (int h = 0; h < G::TBM / 128; ++h)
-            load_slab_cpasync<A_KMAJ>(As + h * 128 * BK, p.A, p.lda, m0 + 128 * h, k0, p.M, p.K,
-                                      lane);
-          load_slab_cpasync<B_KMAJ, G::TBN>(Bs, p.B, p.ldb, n0, k0, p.N, p.K, lane);
+          load_slab_cpasync<A_KMAJ, G::TBM>(As, p.A, p.lda, m0, k0, p.M, p.K, warp & 1, lane);
+          load_slab_cpasync<B_KMAJ, G::TBN>(Bs, p.B, p.ldb, n0, k0, p.N, p.K, warp & 1, lane);
           cp_async_arrive_noinc(&full[s]);
         }
       }
@@ -267,31 +301,44 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   // ------------------------------ consumer warpgroups ------------------------------
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CONSUMER_REGS));
-  const int ct = threadIdx.x - 128;  // consumer thread 0..255
-  const int cw = warp - 4;
-  // 2 x 4 (4 x 2 when narrow) grid of 64 x 32 warp tiles
-  const int wm = cw >> (NARROW ? 1 : 2), wn = cw & (G::WN - 1);
+  const int grp = (warp - 4) >> 2;     // consumer warpgroup, and its ring
+  const int ct = threadIdx.x & 127;     // thread of the warpgroup
+  const int cw = warp & 3;
+  const int w = worker_of(p, grp);
+  uint64_t *full = bars + 2 * STAGES * grp, *empty = full + STAGES;
+  const double *tiles = reinterpret_cast<const double *>(base) + grp * STAGES * STAGE_DBL;
+  const int wm = cw / G::WN, wn = cw % G::WN;  // 64 x 32 warp tile of the unit's tile
   const int g = lane >> 2, t = lane & 3;
-  // Fragment offsets into the swizzled slabs, split into a per-thread part computed once
-  // and compile-time constants (mt, nt, kk).  K-major: element (mn, k) at
-  // mn*16 + 2*((k>>1) ^ (mn&7)) + (k&1), with mn&7 == g and k = kk + t.
-  // MN-major: (mn>>4)*256 + k*16 + 2*(((mn&15)>>1) ^ (k&7)) + (mn&1).
+  // Which row (column) of a 16-wide block of the slab a fragment's index stands for: any
+  // permutation gives the same products as long as the epilogue uses it too, and these make
+  // every fragment load touch all 32 banks once (in plain order two rows 128 bytes apart
+  // meet in the same 16-byte chunk: a two-way conflict on every load).  Index i = 0..7 of
+  // the fragment, h = 0, 1 (rows i and i + 8 of A's fragment; the two 8-column tiles of B):
+  //   K-major : 2 (i & 3) + (i >> 2) + 8 h        MN-major : (i & 1) + 8 (i >> 1 & 1) + 2 (i >> 2) + 4 h
+  // Element (mn, k), k = kk + t, K-major: mn*16 + 2*((k>>1) ^ (mn&7)) + (k&1);
+  // MN-major: (mn>>4)*256 + k*16 + 2*(((mn&15)>>1) ^ (k&7)) + (mn&1).  The offsets are split
+  // into a per-thread part computed once and compile-time constants (mt, nt, kk).
+  const int rk = 2 * (g & 3) + (g >> 2);
   int kv[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) kv[q] = 2 * ((2 * q) ^ (g & 6)) + 2 * ((t >> 1) ^ (g & 1)) + (t & 1);
-  int xa[2][2], xb[2][2];
+  for (int q = 0; q < 4; ++q) kv[q] = 2 * ((2 * q + (t >> 1)) ^ (rk & 7)) + (t & 1);
+  int xa[2][2];
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int q2 = 0; q2 < 2; ++q2) {
-      xa[h][q2] = 2 * (((g >> 1) + 4 * h) ^ (4 * q2 + t));
-      xb[h][q2] = 2 * (((g >> 1) + 4 * h) ^ (4 * q2 + t));
-    }
-  const int a_base = A_KMAJ ? (wm * 64 + g) * 16 : (wm * 4) * 256 + t * 16 + (g & 1);
-  const int b_base = B_KMAJ ? (wn * 32 + g) * 16 : (wn * 2) * 256 + t * 16 + (g & 1);
+    for (int q2 = 0; q2 < 2; ++q2)
+      xa[h][q2] = 2 * ((4 * ((g >> 1) & 1) + (g >> 2) + 2 * h) ^ (4 * q2 + t));
+  const int a_base = A_KMAJ ? (wm * 64 + rk) * 16 : (wm * 4) * 256 + t * 16 + (g & 1);
+  const int b_base =
+      G::TBM * BK + (B_KMAJ ? (wn * 32 + rk) * 16 : (wn * 2) * 256 + t * 16 + (g & 1));
+  // the element of the warp's part of C in accumulator [mt][nt][r]: row fr + 16 mt + RH (r >> 1),
+  // column fc + 16 (nt >> 1) + CH (nt & 1) + CE (r & 1)
+  constexpr int RH = A_KMAJ ? 8 : 4, CH = B_KMAJ ? 8 : 4, CE = B_KMAJ ? 2 : 1;
+  const int fr = A_KMAJ ? rk : (g & 1) + 8 * ((g >> 1) & 1) + 2 * (g >> 2);
+  const int fc = B_KMAJ ? 4 * (t & 1) + (t >> 1) : 8 * (t & 1) + 2 * (t >> 1);
   int it = 0;
   Unit u;
-  for (int ui = 0; unit_at(p, ui, u); ++ui) {
+  for (int ui = 0; unit_at(p, w, ui, u); ++ui) {
     int tm, tn;
     tile_coords(p, u.tile, tm, tn);
     const int m0 = tm * G::TBM, n0 = tn * G::TBN;
@@ -315,120 +362,184 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     // a warp whose 32 columns all lie past N (narrow C, e.g. a residual with few
     // right-hand sides) keeps the stage hand-shake but issues no loads or MMAs
-    const bool idle = n0 + wn * 32 >= p.N;
-    for (int kt = u.k0; kt < u.k1; ++kt, ++it) {
-      const int s = it % STAGES;
-      const uint32_t ph = (it / STAGES) & 1;
-      if (!mbar_wait(&full[s], ph, p.status)) return;
-      const double *As = tiles + s * G::STAGE_DBL;
-      const double *Bs = As + G::A_DBL;
+    const bool idle = n0 + wn * 32 >= p.N || m0 + wm * 64 >= p.M;
+    // fragments of k-step kk = 4 q of the slab at `st`
+    auto load_frag = [&](const double *st, int q, double (&a)[4][2], double (&b)[4]) {
+      const int q2 = q & 1, kk = 4 * q;
 #pragma unroll
-      for (int kk = 0; kk < BK && !idle; kk += 4) {
-        const int q = kk >> 2, q2 = q & 1;
-        double a[4][2], b[4];
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-          if constexpr (A_KMAJ) {
-            a[mt][0] = As[a_base + kv[q] + mt * 256];
-            a[mt][1] = As[a_base + kv[q] + mt * 256 + 128];
-          } else {
-            a[mt][0] = As[a_base + xa[0][q2] + mt * 256 + kk * 16];
-            a[mt][1] = As[a_base + xa[1][q2] + mt * 256 + kk * 16];
-          }
+      for (int mt = 0; mt < 4; ++mt) {
+        if constexpr (A_KMAJ) {
+          a[mt][0] = st[a_base + kv[q] + mt * 256];
+          a[mt][1] = st[a_base + kv[q] + mt * 256 + 128];
+        } else {
+          a[mt][0] = st[a_base + xa[0][q2] + mt * 256 + kk * 16];
+          a[mt][1] = st[a_base + xa[1][q2] + mt * 256 + kk * 16];
         }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          if constexpr (B_KMAJ)
-            b[nt] = Bs[b_base + kv[q] + nt * 128];
-          else
-            b[nt] = Bs[b_base + xb[nt & 1][q2] + (nt >> 1) * 256 + kk * 16];
-        }
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        if constexpr (B_KMAJ)
+          b[nt] = st[b_base + kv[q] + nt * 128];
+        else
+          b[nt] = st[b_base + xa[nt & 1][q2] + (nt >> 1) * 256 + kk * 16];
+      }
+    };
+    const int nk = u.k1 - u.k0;
+    // two or more whole tiles each: warpgroup 1 starts half a tile after warpgroup 0
+    const bool stagger = ui == 0 && p.dp_tiles > p.workers && nk > 0;
+    if (stagger && grp == 1 && !mbar_wait(late, 0, p.status)) return;
+    const int half = stagger && grp == 0 ? nk / 2 : -1;
+    if (idle) {
+      for (int kt = 0; kt < nk; ++kt, ++it) {
+        const int s = it % STAGES;
+        if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status)) return;
+        if (lane == 0) {
+          mbar_arrive(&empty[s]);
+          if (kt == half) mbar_arrive(late);
+        }
+      }
+    } else {
+      for (int kt = 0; kt < nk; ++kt, ++it) {
+        const int s = it % STAGES;
+        if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status)) return;
+        const double *st = tiles + s * STAGE_DBL;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          double a[4][2], b[4];
+          load_frag(st, q, a, b);
+#pragma unroll
+          for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&empty[s]);
+          if (kt == half) mbar_arrive(late);
+        }
+      }
     }
 
     if (!u.owner) {
-      // publish the partial sum (fragment order: register r of consumer thread ct at
-      // [r * 256 + ct], coalesced per warp), then stamp this CTA's flag
-      double *slot = p.partial + (size_t)blockIdx.x * (64 * 256);
+      // publish the partial sum (fragment order: register r of thread ct at
+      // [r * 128 + ct], coalesced per warp), then stamp this worker's flag
+      double *slot = p.partial + (size_t)w * TILE_DBL;
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-          for (int r = 0; r < 4; ++r) slot[((mt * 4 + nt) * 4 + r) * 256 + ct] = acc[mt][nt][r];
+          for (int r = 0; r < 4; ++r) slot[((mt * 4 + nt) * 4 + r) * 128 + ct] = acc[mt][nt][r];
       __threadfence();
-      consumer_bar();
-      if (ct == 0) atomicExch(&p.flags[blockIdx.x], p.epoch);
+      group_bar(grp);
+      if (ct == 0) atomicExch(&p.flags[w], p.epoch);
       continue;
     }
-    if (u.first_contrib < (int)blockIdx.x) {
-      // add the partials of the lower-numbered CTAs that computed the tile's first slabs
-      for (int c = u.first_contrib; c < (int)blockIdx.x; ++c) {
+    if (u.first_contrib < w) {
+      // add the partials of the lower-numbered workers that computed the tile's first slabs
+      for (int c = u.first_contrib; c < w; ++c) {
         if (ct == 0) {
           uint32_t i = 0;
           while (atomicAdd(&p.flags[c], 0) != p.epoch) {
             if (++i > MO_SPIN_LIMIT) {
               set_status(p.status, MO_EDEVTIMEOUT);
-              s_abort = 1;
+              s_abort[grp] = 1;
               break;
             }
           }
           __threadfence();
         }
-        consumer_bar();
-        if (s_abort) return;
-        const double *slot = p.partial + (size_t)c * (64 * 256);
+        group_bar(grp);
+        if (s_abort[grp]) return;
+        const double *slot = p.partial + (size_t)c * TILE_DBL;
 #pragma unroll
         for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
           for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int r = 0; r < 4; ++r)
-              acc[mt][nt][r] += __ldcg(slot + ((mt * 4 + nt) * 4 + r) * 256 + ct);
+              acc[mt][nt][r] += __ldcg(slot + ((mt * 4 + nt) * 4 + r) * 128 + ct);
       }
     }
 
     // ------------------------------ epilogue ------------------------------
-    // 16 elements at a time: all loads of C are issued before any store, so the L2 round
-    // trips overlap (stores may alias later loads, which would otherwise serialize them)
     // C is read unless beta == 0 everywhere (with diagonal-block beta, off-block
-    // elements use beta = 1)
+    // elements use beta = 1).  All loads of a batch are issued before any store, so the L2
+    // round trips overlap (stores may alias later loads, which would otherwise serialize
+    // them).
     const bool need_c = p.beta != 0.0 || p.beta_block > 0;
+    const int wr = m0 + wm * 64, wc = n0 + wn * 32;  // the warp's 64 x 32 part of C
+    bool whole = wr + 64 <= p.M && wc + 32 <= p.N && p.beta_block == 0;
+    if (p.mode == kSyrkLower || p.mode == kGemmLower) whole = whole && wr >= wc + 31;
+    if (p.mode == kSyrkUpper || p.mode == kGemmUpper) whole = whole && wr + 63 <= wc;
+    if (whole) {
+      // every element is kept and has the same beta: no tests per element.  (With the tests
+      // and their branches on all 64 elements the epilogue took as long as 85 columns of K.)
+      const double alpha = p.alpha, beta = p.beta;
+      double *cp[4];
+      cp[0] = p.C + (wr + fr) + (int64_t)(wc + fc) * p.ldc;
+      cp[1] = cp[0] + CH * p.ldc;
+      cp[2] = cp[0] + 16 * p.ldc;
+      cp[3] = cp[2] + CH * p.ldc;
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+        if (beta != 0.0) {
+          double cv[4][4];
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              cv[nt][r] = __ldcg(cp[nt] + mt * 16 + RH * (r >> 1) + CE * (r & 1) * p.ldc);
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              cp[nt][mt * 16 + RH * (r >> 1) + CE * (r & 1) * p.ldc] =
+                  fma(beta, cv[nt][r], alpha * acc[mt][nt][r]);
+        } else {
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              cp[nt][mt * 16 + RH * (r >> 1) + CE * (r & 1) * p.ldc] = alpha * acc[mt][nt][r];
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (int mt = 0; mt < 4; ++mt) {
-      double cv[4][4];
-      bool keep[4][4];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+      for (int nh = 0; nh < 4; nh += 2) {
+        double cv[2][4];
+        const int row0 = wr + fr + mt * 16, col0 = wc + fc + nh * 8;
+        double *c0 = p.C + row0 + (int64_t)col0 * p.ldc;
+        unsigned keep = 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = m0 + wm * 64 + mt * 16 + g + ((r >> 1) << 3);
-          const int col = n0 + wn * 32 + nt * 8 + 2 * t + (r & 1);
-          bool k = row < p.M && col < p.N;
-          if ((p.mode == kSyrkLower || p.mode == kGemmLower) && row < col) k = false;
-          if ((p.mode == kSyrkUpper || p.mode == kGemmUpper) && row > col) k = false;
-          keep[nt][r] = k;
-          cv[nt][r] = (k && need_c) ? __ldcg(p.C + row + (int64_t)col * p.ldc) : 0.0;
-        }
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+          for (int r = 0; r < 4; ++r) {
+            const int row = row0 + RH * (r >> 1), col = col0 + CH * nt + CE * (r & 1);
+            bool k = row < p.M && col < p.N;
+            if ((p.mode == kSyrkLower || p.mode == kGemmLower) && row < col) k = false;
+            if ((p.mode == kSyrkUpper || p.mode == kGemmUpper) && row > col) k = false;
+            keep |= (k ? 1u : 0u) << (nt * 4 + r);
+            cv[nt][r] = (k && need_c)
+                            ? __ldcg(c0 + RH * (r >> 1) + (int64_t)(CH * nt + CE * (r & 1)) * p.ldc)
+                            : 0.0;
+          }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          if (!keep[nt][r]) continue;
-          const int row = m0 + wm * 64 + mt * 16 + g + ((r >> 1) << 3);
-          const int col = n0 + wn * 32 + nt * 8 + 2 * t + (r & 1);
-          double bet = p.beta;
-          if (p.beta_block > 0 && (row / p.beta_block) != (col / p.beta_block)) bet = 1.0;
-          double v = p.alpha * acc[mt][nt][r];
-          if (bet != 0.0) v = fma(bet, cv[nt][r], v);
-          p.C[row + (int64_t)col * p.ldc] = v;
-        }
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            if (!(keep >> (nt * 4 + r) & 1u)) continue;
+            const int row = row0 + RH * (r >> 1), col = col0 + CH * nt + CE * (r & 1);
+            double bet = p.beta;
+            if (p.beta_block > 0 && (row / p.beta_block) != (col / p.beta_block)) bet = 1.0;
+            double v = p.alpha * acc[mt][nh + nt][r];
+            if (bet != 0.0) v = fma(bet, cv[nt][r], v);
+            c0[RH * (r >> 1) + (int64_t)(CH * nt + CE * (r & 1)) * p.ldc] = v;
+          }
+      }
     }
   }
 }
@@ -465,11 +576,10 @@ bool make_tmap(CUtensorMap *tm, const double *ptr, uint64_t inner, uint64_t oute
   return r == CUDA_SUCCESS;
 }
 
-template <bool AK, bool BKM, bool TMA, bool NARROW>
+template <bool AK, bool BKM, bool TMA, bool WIDE>
 int launch_inst(const KParams &kp, const CUtensorMap &ta, const CUtensorMap &tb, int grid,
                 cudaStream_t st) {
-  constexpr int SMEM_BYTES = Geo<NARROW>::SMEM;
-  auto kern = dgemm_tile_kernel<AK, BKM, TMA, NARROW>;
+  auto kern = dgemm_tile_kernel<AK, BKM, TMA, WIDE>;
   // setmaxnreg.inc only draws on the registers the CTA was launched with: refuse to launch
   // (instead of waiting forever) if the build did not keep the 168-register split (a
   // property of the binary, checked once)
@@ -488,13 +598,13 @@ int launch_inst(const KParams &kp, const CUtensorMap &ta, const CUtensorMap &tb,
   return MO_OK;
 }
 
-template <bool TMA, bool NARROW>
+template <bool TMA, bool WIDE>
 int dispatch(bool ak, bool bk, const KParams &kp, const CUtensorMap &ta, const CUtensorMap &tb,
              int grid, cudaStream_t st) {
-  if (ak) return bk ? launch_inst<true, true, TMA, NARROW>(kp, ta, tb, grid, st)
-                    : launch_inst<true, false, TMA, NARROW>(kp, ta, tb, grid, st);
-  return bk ? launch_inst<false, true, TMA, NARROW>(kp, ta, tb, grid, st)
-            : launch_inst<false, false, TMA, NARROW>(kp, ta, tb, grid, st);
+  if (ak) return bk ? launch_inst<true, true, TMA, WIDE>(kp, ta, tb, grid, st)
+                    : launch_inst<true, false, TMA, WIDE>(kp, ta, tb, grid, st);
+  return bk ? launch_inst<false, true, TMA, WIDE>(kp, ta, tb, grid, st)
+            : launch_inst<false, false, TMA, WIDE>(kp, ta, tb, grid, st);
 }
 
 }  // namespace
@@ -504,8 +614,7 @@ bool gemm_tma_ok(const GemmArgs &a) {
   return al(a.A) && al(a.B) && (a.lda % 2 == 0) && (a.ldb % 2 == 0) && encode_fn() != nullptr;
 }
 
-int gemm_partial_slots(int sms) { return sms; }
-size_t gemm_partial_bytes(int sms) { return (size_t)sms * 64 * 256 * sizeof(double); }
+size_t gemm_partial_bytes(int sms) { return 2 * (size_t)sms * TILE_DBL * sizeof(double); }
 
 int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0) return MO_OK;
@@ -525,9 +634,13 @@ int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
   kp.beta_block = a.beta_block;
   kp.status = a.status;
   kp.skip = a.skip;
-  // narrow C (a residual with few right-hand sides): 256 x 64 tiles
-  const bool narrow = a.mode == kGemm && a.N <= 64 && a.M >= 2048;
-  const int tbm = narrow ? Geo<true>::TBM : BM, tbn = narrow ? Geo<true>::TBN : BN;
+  // 64 x 128 tiles for C = op(A) itself (each tile then reads and writes its own rows
+  // only; N <= 128 there) and for a C of at most 64 rows; 128 x 64 otherwise, which also
+  // is the shape of in-place products from the left (C = op(B), M <= 128)
+  const bool wide =
+      a.mode == kGemm && (a.C == a.A || (a.M <= 64 && a.N > 64 && a.C != a.B));
+  const int tbm = wide ? Geo<true>::TBM : Geo<false>::TBM;
+  const int tbn = wide ? Geo<true>::TBN : Geo<false>::TBN;
   const int tiles_m = (a.M + tbm - 1) / tbm, tiles_n = (a.N + tbn - 1) / tbn;
   kp.tiles_m = tiles_m;
   kp.tiles_n = tiles_n;
@@ -536,63 +649,66 @@ int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
     T = (long long)tiles_m * tiles_n;
   } else {
     if (a.M != a.N) return MO_EINVAL;
-    T = (long long)tiles_m * (tiles_m + 1) / 2;
+    T = (long long)tiles_m * (tiles_m + 1);  // two tiles per 128 x 128 square
   }
   if (T <= 0 || T > 0x7fffffffLL) return MO_EINVAL;
   kp.total_tiles = (int)T;
   kp.kt = (kp.K + BK - 1) / BK;
   int sms = a.sms > 0 ? a.sms : 148;
   if (a.max_ctas > 0 && a.max_ctas < sms) sms = a.max_ctas;
-  // Schedule: whole tiles round-robin over persistent CTAs; when a GEMM has only a few,
-  // unequal waves (e.g. 256 tiles on 148 SMs), the last one or two waves are split along
-  // K evenly over all CTAs (stream-K) and finished by the CTA holding each tile's last slab.
-  int grid = (int)std::min<long long>(T, sms);
+  // Schedule: whole tiles round-robin over the workers (two per CTA) of a persistent grid;
+  // when a GEMM has only a few, unequal waves (e.g. 512 tiles on 2 x 148 workers), the last
+  // one or two waves are split along K evenly over all workers (stream-K) and finished by
+  // the worker holding each tile's last slab.
+  const int slots = 2 * sms;
+  kp.workers = (int)std::min<long long>(T, slots);
   kp.dp_tiles = (int)T;
   kp.sk_iters = 0;
   kp.sk_chunk = 1;
   kp.partial = a.sk_partial;
   kp.flags = a.sk_flags;
   kp.epoch = a.sk_epoch;
-  const long long waves = T / sms, rem = T % sms;
+  const long long waves = T / slots, rem = T % slots;
   if (a.mode == kGemm && a.sk_partial && a.sk_flags && rem != 0 && waves < 4 && kp.kt >= 8) {
-    const long long dp = (waves >= 1 ? waves - 1 : 0) * sms;
+    const long long dp = (waves >= 1 ? waves - 1 : 0) * slots;
     kp.dp_tiles = (int)dp;
     kp.sk_iters = (int)((T - dp) * kp.kt);
-    grid = sms;
-    kp.sk_chunk = (kp.sk_iters + grid - 1) / grid;
+    kp.workers = slots;
+    kp.sk_chunk = (kp.sk_iters + slots - 1) / slots;
     if (kp.sk_chunk < 4) {
-      // too little work for every CTA: fewer CTAs with 4 slabs each when that still uses
-      // more SMs than whole tiles would (a few tiles with a long K, e.g. one 128 x 128
-      // tile with K in the thousands), else data-parallel
+      // too little work for every worker: fewer workers with 4 slabs each when that still
+      // uses more of them than whole tiles would (a few tiles with a long K, e.g. one
+      // 128 x 128 block with K in the thousands), else data-parallel
       const long long g2 = kp.sk_iters / 4;
       if (kp.kt >= 32 && g2 > T) {
-        grid = (int)std::min<long long>(g2, sms);
-        kp.sk_chunk = (kp.sk_iters + grid - 1) / grid;
+        kp.workers = (int)std::min<long long>(g2, slots);
+        kp.sk_chunk = (kp.sk_iters + kp.workers - 1) / kp.workers;
       } else {
         kp.dp_tiles = (int)T;
         kp.sk_iters = 0;
         kp.sk_chunk = 1;
-        grid = (int)std::min<long long>(T, sms);
+        kp.workers = (int)std::min<long long>(T, slots);
       }
     }
   }
+  const int grid = std::min(kp.workers, sms);
 
   const bool ak = a.transA;   // op(A) stored K-major when A is transposed
   const bool bk = !a.transB;  // op(B) stored K-major when B is not transposed
   CUtensorMap ta, tb;
   const bool use_tma = !a.force_fallback && kp.K > 0 && gemm_tma_ok(a);
   if (use_tma) {
-    bool okA = ak ? make_tmap(&ta, a.A, kp.K, a.M, a.lda, 16, 128)
+    bool okA = ak ? make_tmap(&ta, a.A, kp.K, a.M, a.lda, 16, (uint32_t)tbm)
                   : make_tmap(&ta, a.A, a.M, kp.K, a.lda, 16, 16);
     bool okB = bk ? make_tmap(&tb, a.B, kp.K, a.N, a.ldb, 16, (uint32_t)tbn)
                   : make_tmap(&tb, a.B, a.N, kp.K, a.ldb, 16, 16);
     if (okA && okB)
-      return narrow ? dispatch<true, true>(ak, bk, kp, ta, tb, grid, stream)
+      return wide ? dispatch<true, true>(ak, bk, kp, ta, tb, grid, stream)
                     : dispatch<true, false>(ak, bk, kp, ta, tb, grid, stream);
   }
   memset(&ta, 0, sizeof(ta));
   memset(&tb, 0, sizeof(tb));
-  return narrow ? dispatch<false, true>(ak, bk, kp, ta, tb, grid, stream)
+  return wide ? dispatch<false, true>(ak, bk, kp, ta, tb, grid, stream)
                 : dispatch<false, false>(ak, bk, kp, ta, tb, grid, stream);
 }
 

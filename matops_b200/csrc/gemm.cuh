@@ -34,8 +34,8 @@ struct GemmArgs {
   bool force_fallback = false;  // use the cp.async producer even when TMA is legal
   int sms = 148;                // persistent grid size
   int max_ctas = 0;             // > 0: cap the persistent grid (leave SMs to other streams)
-  // stream-K scratch (nullptr: data-parallel schedule only): one 128 KB partial-sum slot
-  // and one flag per CTA, and a value unique to this launch for the flags
+  // stream-K scratch (nullptr: data-parallel schedule only): two 64 KB partial-sum slots
+  // and two flags per CTA, and a value unique to this launch for the flags
   double *sk_partial = nullptr;
   int *sk_flags = nullptr;
   int sk_epoch = 0;
