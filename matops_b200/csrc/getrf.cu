@@ -6,10 +6,12 @@
 // first row holding the strict maximum of |x|; a NaN never wins unless it sits on the
 // diagonal, where the scan starts).  The factors do not depend on left- vs right-looking
 // order except through rounding, so the device runs the right-looking form:
-//   panel   : cooperative kernel, every CTA owns a slice of panel rows in shared memory,
-//             one grid barrier per column (candidate rows are published with the local
-//             argmax, so every CTA picks the pivot itself)
-//   laswp   : apply the panel's interchanges to the columns left and right of it
+//   panel   : up to 16384 rows one thread-block cluster, rows in registers, one cluster
+//             barrier per column; above, a cooperative kernel whose CTAs own slices of the
+//             panel in shared memory, one grid barrier per column (candidate rows are
+//             published with the local argmax, so every CTA picks the pivot itself)
+//   laswp   : apply the panel's interchanges to the other columns (all of them after the
+//             cluster panel, which leaves its rows where they were)
 //   trsm    : U12 = L11^-1 A12 (unit lower inverse + in-place GEMM)
 //   update  : A22 -= L21 U12 on the FP64 tensor pipe
 #include <algorithm>
@@ -241,6 +243,417 @@ __global__ void __launch_bounds__(PANEL_THREADS)
     const int r = e % nr, c = e / nr;
     P[(rbeg + r) + (int64_t)c * ld] = S[r * LDW + c];
   }
+}
+
+// ---- the panel in one thread-block cluster ---------------------------------------------
+// What bounds a panel is its chain of columns: pivot search, exchange of the pivot row,
+// scaling, update, and nothing of column j + 1 can start before.  A grid barrier costs
+// several L2 round trips per column (5.0 us a column with the cooperative kernel below at
+// 1001 and at 16384 rows); inside a cluster the candidates travel through distributed shared
+// memory and one hardware barrier.  16 CTAs x 512 threads x 2 rows hold 16384 rows of a
+// 16-column sub-panel in registers; the 128 columns are done left-looking, sub-panel by
+// sub-panel: a thread first applies the finished columns to its rows (L from L2, U from
+// shared memory), then the 16 columns are eliminated.  Every entry takes the same FMAs in
+// the same order as in a right-looking panel.
+//
+// Rows do not move in memory: a thread holds a logical row and its physical row, an
+// interchange exchanges both between two threads, and the moves that put all columns of the
+// matrix (the panel's among them) in order are emitted at the end.
+//
+// Measured on B200, 128 columns with the interchanges applied, against the cooperative
+// kernel: 128 rows 608 -> 187 us, 1001 rows 671 -> 256, 4000 rows 698 -> 264, 8000 rows 708 ->
+// 320, 16000 rows 766 -> 439 (there the FP64 rate of the 16 SMs takes over).  A column takes
+// about 1000 cycles in one CTA and 1700 in a cluster, half of it the two argmax levels and
+// the exchange; the triangle of U and the left-looking products take the other third.
+constexpr int kClThreads = 256, kClWarps = kClThreads / 32, kClSub = 16, kClMaxCtas = 16;
+constexpr int kClMaxRows = kClThreads * kClMaxCtas * 4;
+constexpr int kClL = MAX_PANEL_W - kClSub;  // rows of U that a later sub-panel needs
+constexpr int kClLd = kClL + 2;  // a row of L^T (16-byte aligned, 4 banks from the next)
+
+struct __align__(16) ClRow {
+  double x[kClSub];       // the row's columns from the current one on
+  unsigned hi, lo;        // key: bits of |x_0|
+  int idx, phys;          // logical and physical row
+};
+
+struct ClSmem {
+  uint64_t bar[2];            // arrival of a column's packets, by column parity
+  uint64_t pad[2];
+  ClRow recv[2][kClMaxCtas];  // one candidate per CTA, double-buffered by column
+  ClRow rowj[2];              // the row at the diagonal
+  ClRow own;                  // this CTA's candidate, gathered for sending
+  ClRow ownj;                 // (CTA 0) the diagonal row, gathered for sending
+  unsigned red_hi[2][kClWarps], red_lo[2][kClWarps];
+  int red_idx[2][kClWarps];
+  int phys[MAX_PANEL_W];      // (CTA 0) physical rows of the logical rows < W
+  __align__(16) double U[kClL * kClSub];    // finished rows of the current 16 columns
+  __align__(16) double L[(kClL + 1) * kClLd];  // (CTA 0) finished rows of L, transposed
+};
+
+__device__ __forceinline__ uint32_t cl_map(const void *p, int cta) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
+}
+// `src` (this CTA's shared memory) to the same place `dst` of every CTA of the cluster, the
+// bytes counted on that CTA's barrier `bar`: the calling warp's lane pair (2 c, 2 c + 1)
+// writes CTA c's copy, nine 16-byte pieces in all.  (Plain remote stores need a cluster
+// barrier with release semantics, which also waits for the multipliers' global stores: 1330
+// cycles a column.)
+__device__ __forceinline__ void cl_send(ClRow *dst, const ClRow *src, uint64_t *bar, int lane,
+                                        int nctas) {
+  const int c = lane >> 1;
+  if (c >= nctas) return;
+  const uint32_t to = cl_map(dst, c), mb = cl_map(bar, c);
+  const double2 *s = reinterpret_cast<const double2 *>(src);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const int p = 2 * i + (lane & 1);
+    if (p < 9) {
+      const double2 v = s[p];
+      asm volatile(
+          "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
+              to + 16 * p),
+          "d"(v.x), "d"(v.y), "r"(mb)
+          : "memory");
+    }
+  }
+}
+static_assert(sizeof(ClRow) == 9 * 16, "row packet");
+static_assert(kClThreads == kClSub * kClSub && kClThreads >= MAX_PANEL_W, "index splits below");
+
+// warp-wide largest key, lowest index on ties; every lane gets the result
+__device__ __forceinline__ void cl_argmax(unsigned &hi, unsigned &lo, int &idx) {
+  const unsigned h = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
+  idx = (int)__reduce_min_sync(0xffffffffu, hi == h && lo == l ? (unsigned)idx : (unsigned)INT_MAX);
+  hi = h;
+  lo = l;
+}
+
+template <int RPT>
+__global__ void __launch_bounds__(kClThreads, 1)
+    lu_cluster_panel_kernel(double *P, int64_t ld, int m, int W, int64_t *piv, int64_t row0,
+                            double *ubuf, int *mv_dst, int *mv_src, int *mv_count,
+                            int *status) {
+  extern __shared__ __align__(16) unsigned char cl_raw[];
+  ClSmem &s = *reinterpret_cast<ClSmem *>(cl_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nctas = gridDim.x, cta = blockIdx.x;  // one cluster: the grid is the cluster
+  const int rbase = cta * kClThreads * RPT + tid;  // logical rows rbase + kClThreads q
+  int phys[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) phys[q] = rbase + kClThreads * q;
+  if (cta == 0 && tid == 0) *mv_count = W;
+  if (tid == 0) {
+    mbar_init(&s.bar[0], 1);
+    mbar_init(&s.bar[1], 1);
+    fence_barrier_init();
+  }
+  if (nctas > 1) cl_sync();  // every CTA has started before any writes into its memory
+  for (int j0 = 0; j0 < W; j0 += kClSub) {
+    const int w = min(kClSub, W - j0);
+    double x[RPT][kClSub];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+#pragma unroll
+      for (int k = 0; k < kClSub; ++k)
+        x[q][k] = (rbase + kClThreads * q < m && k < w)
+                      ? __ldcg(P + phys[q] + (int64_t)(j0 + k) * ld) : 0.0;
+    // LB columns of L of this thread's unfinished rows
+    constexpr int LB = 8 / RPT;
+    double l0[RPT][LB], l1[RPT][LB];
+    auto fetch = [&](int i0, double (&l)[RPT][LB]) {
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        const int r = rbase + kClThreads * q;
+        const double *src = P + phys[q] + (int64_t)i0 * ld;
+#pragma unroll
+        for (int i = 0; i < LB; ++i) l[q][i] = r >= j0 && r < m ? __ldcg(src + i * ld) : 0.0;
+      }
+    };
+    if (j0 > 0) {
+      fetch(0, l0);
+      // rows < j0 of these columns: U = L^-1 A by CTA 0, 16 rows at a time
+      if (cta == 0) {
+        {  // the 16 newest rows of L, all loads in flight at once
+          const int i = j0 - kClSub + (tid & (kClSub - 1)), k1 = tid / kClSub;
+          const double *src = P + s.phys[i];
+          double v[kClL / kClSub];
+#pragma unroll
+          for (int n = 0; n < kClL / kClSub; ++n) {
+            const int k = k1 + kClSub * n;
+            v[n] = k < i ? __ldcg(src + (int64_t)k * ld) : 0.0;
+          }
+#pragma unroll
+          for (int n = 0; n < kClL / kClSub; ++n) s.L[(k1 + kClSub * n) * kClLd + i] = v[n];
+        }
+        if (tid < j0) {
+#pragma unroll
+          for (int k = 0; k < kClSub; ++k) s.U[tid * kClSub + k] = x[0][k];
+        }
+        __syncthreads();
+        const int c = tid & (kClSub - 1), i1 = tid / kClSub;
+        for (int b = 0; b < j0; b += kClSub) {
+          if (tid < kClSub) {  // 16 x 16 unit lower triangle, one thread per column
+            double u[kClSub];
+#pragma unroll
+            for (int i = 0; i < kClSub; ++i) u[i] = s.U[(b + i) * kClSub + tid];
+#pragma unroll
+            for (int k = 0; k + 1 < kClSub; ++k) {
+              const double2 *lk = reinterpret_cast<const double2 *>(s.L + (b + k) * kClLd + b);
+#pragma unroll
+              for (int i2 = (k + 1) / 2; i2 < kClSub / 2; ++i2) {
+                const double2 v = lk[i2];
+                if (2 * i2 > k) u[2 * i2] = fma(-v.x, u[k], u[2 * i2]);
+                u[2 * i2 + 1] = fma(-v.y, u[k], u[2 * i2 + 1]);
+              }
+            }
+#pragma unroll
+            for (int i = 1; i < kClSub; ++i) s.U[(b + i) * kClSub + tid] = u[i];
+          }
+          __syncthreads();
+          // the rows below it, 16 at a time by all threads, all of a thread's rows together
+          // (those past j0 compute on what the padded array holds and are not stored)
+          double a[kClL / kClSub - 1];
+          const int nr = (j0 - b) / kClSub - 1;
+#pragma unroll
+          for (int j = 0; j < kClL / kClSub - 1; ++j)
+            a[j] = j < nr ? s.U[(b + kClSub * (j + 1) + i1) * kClSub + c] : 0.0;
+#pragma unroll
+          for (int k = 0; k < kClSub; ++k) {
+            const double uk = s.U[(b + k) * kClSub + c];
+            const double *lk = s.L + (b + k) * kClLd + b + kClSub + i1;
+#pragma unroll
+            for (int j = 0; j < kClL / kClSub - 1; ++j) a[j] = fma(-lk[kClSub * j], uk, a[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < kClL / kClSub - 1; ++j)
+            if (j < nr) s.U[(b + kClSub * (j + 1) + i1) * kClSub + c] = a[j];
+          __syncthreads();
+        }
+        for (int e = tid; e < kClSub * j0; e += kClThreads) {
+          const int i = e % j0, k = e / j0;
+          if (k < w) P[s.phys[i] + (int64_t)(j0 + k) * ld] = s.U[i * kClSub + k];
+        }
+        if (nctas > 1)
+          for (int e = tid; e < j0 * kClSub; e += kClThreads) ubuf[e] = s.U[e];
+      }
+      if (nctas > 1) {
+        cl_sync();
+        if (cta != 0) {
+          for (int e = tid; e < j0 * kClSub; e += kClThreads) s.U[e] = __ldcg(ubuf + e);
+          __syncthreads();
+        }
+      }
+      // rows >= j0 take the finished columns, a batch of them while the next batch's L is on
+      // its way (the first one was requested before U)
+      auto apply = [&](int i0, const double (&l)[RPT][LB]) {
+#pragma unroll
+        for (int i = 0; i < LB; ++i) {
+          const double2 *u = reinterpret_cast<const double2 *>(s.U + (i0 + i) * kClSub);
+#pragma unroll
+          for (int k = 0; k < kClSub / 2; ++k) {
+            const double2 v = u[k];
+#pragma unroll
+            for (int q = 0; q < RPT; ++q) {
+              x[q][2 * k] = fma(-l[q][i], v.x, x[q][2 * k]);
+              x[q][2 * k + 1] = fma(-l[q][i], v.y, x[q][2 * k + 1]);
+            }
+          }
+        }
+      };
+#pragma unroll 1
+      for (int i0 = 0; i0 < j0; i0 += 2 * LB) {
+        fetch(i0 + LB, l1);
+        apply(i0, l0);
+        if (i0 + 2 * LB < j0) fetch(i0 + 2 * LB, l0);
+        apply(i0 + LB, l1);
+      }
+    }
+    // Eliminate the columns.  The loop is rolled (the registers shift by one column per turn:
+    // x[q][0] is always the current one): with the 16 columns unrolled every instruction
+    // ran once per sub-panel and the fetches, not the arithmetic, set the time.  A finished
+    // multiplier goes straight to its physical row in memory.
+    unsigned hi = 0, lo = 0;
+    int idx = INT_MAX;
+    // this thread's largest |x_0| among the rows >= jc (pivot.go:98-107): first index of the
+    // maximum; a NaN wins only on the diagonal, where its bits exceed every number's
+    auto search = [&](int jc) {
+      hi = lo = 0u;
+      idx = INT_MAX;
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        const int r = rbase + kClThreads * q;
+        const unsigned long long bits = __double_as_longlong(fabs(x[q][0]));
+        const bool nan = bits > 0x7ff0000000000000ull && r != jc;
+        const unsigned h2 = nan ? 0u : (unsigned)(bits >> 32), l2 = nan ? 0u : (unsigned)bits;
+        if (r >= jc && r < m && (idx == INT_MAX || h2 > hi || (h2 == hi && l2 > lo))) {
+          hi = h2;
+          lo = l2;
+          idx = r;
+        }
+      }
+    };
+    search(j0);
+#pragma unroll 1
+    for (int c = 0; c < w; ++c) {
+      const int jc = j0 + c, par = jc & 1;
+      // this column's packets: one candidate per CTA and the diagonal row
+      if (nctas > 1 && tid == 0)
+        mbar_arrive_expect_tx(&s.bar[par], (uint32_t)((nctas + 1) * sizeof(ClRow)));
+      cl_argmax(hi, lo, idx);
+      if (lane == 0) {
+        s.red_hi[par][warp] = hi;
+        s.red_lo[par][warp] = lo;
+        s.red_idx[par][warp] = idx;
+      }
+      // the diagonal row (always one of CTA 0's first rows) goes out beside the search
+      if (cta == 0 && warp == jc / 32) {
+        ClRow &to = nctas > 1 ? s.ownj : s.rowj[par];
+        if (tid == jc) {
+#pragma unroll
+          for (int k = 0; k < kClSub; ++k) to.x[k] = x[0][k];
+          to.phys = phys[0];
+        }
+        __syncwarp();
+        if (nctas > 1) cl_send(&s.rowj[par], &s.ownj, &s.bar[par], lane, nctas);
+      }
+      __syncthreads();
+      hi = s.red_hi[par][lane & (kClWarps - 1)];
+      lo = s.red_lo[par][lane & (kClWarps - 1)];
+      idx = s.red_idx[par][lane & (kClWarps - 1)];
+      cl_argmax(hi, lo, idx);
+      // this CTA's candidate, from its owner's registers to every CTA
+      if (warp == (idx == INT_MAX ? 0 : (idx & (kClThreads - 1)) >> 5)) {
+        ClRow &to = nctas > 1 ? s.own : s.recv[par][0];
+        if (idx == INT_MAX && lane == 0) {  // no row left in this CTA
+          to.hi = to.lo = 0u;
+          to.idx = INT_MAX;
+        }
+#pragma unroll
+        for (int q = 0; q < RPT; ++q)
+          if (rbase + kClThreads * q == idx) {
+#pragma unroll
+            for (int k = 0; k < kClSub; ++k) to.x[k] = x[q][k];
+            to.hi = hi;
+            to.lo = lo;
+            to.idx = idx;
+            to.phys = phys[q];
+          }
+        __syncwarp();
+        if (nctas > 1) cl_send(&s.recv[par][cta], &s.own, &s.bar[par], lane, nctas);
+      }
+      // every warp picks the pivot: largest key, lowest row
+      if (nctas > 1) {
+        // (a wait that runs out is recorded; the kernel goes on with what it holds)
+        mbar_wait(&s.bar[par], (jc >> 1) & 1, status);
+        const ClRow &cand = s.recv[par][lane < nctas ? lane : 0];
+        hi = cand.hi;
+        lo = cand.lo;
+        idx = cand.idx;
+        cl_argmax(hi, lo, idx);
+      } else {
+        __syncthreads();
+      }
+      const int p = min(max(idx, jc), m - 1);  // (idx itself, unless a wait ran out)
+      const ClRow &pr = s.recv[par][p / (kClThreads * RPT)];
+      double u[kClSub];
+#pragma unroll
+      for (int k = 0; k < kClSub / 2; ++k) {
+        const double2 v = reinterpret_cast<const double2 *>(pr.x)[k];
+        u[2 * k] = v.x;
+        u[2 * k + 1] = v.y;
+      }
+      if (cta == 0 && warp == kClWarps - 1) {  // the U row, and the pivot
+        if (lane < w - c)
+          P[min(max(pr.phys, 0), m - 1) + (int64_t)(jc + lane) * ld] = pr.x[lane];
+        if (lane == 0) piv[jc] = row0 + p;
+      }
+      if (p != jc && (warp == ((p & (kClThreads - 1)) >> 5) || warp == jc / 32)) {
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          const int r = rbase + kClThreads * q;
+          if (r == p) {
+#pragma unroll
+            for (int k = 0; k < kClSub; ++k) x[q][k] = s.rowj[par].x[k];
+            phys[q] = min(max(s.rowj[par].phys, 0), m - 1);
+          } else if (r == jc) {
+            phys[q] = min(max(pr.phys, 0), m - 1);
+          }
+        }
+      }
+      // l = a / u (true division, mvec.go:422 InvScale) and the rank-1 update, on every row
+      // (the rows <= jc hold nothing that is read again)
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        const int r = rbase + kClThreads * q;
+        const double l = x[q][0] / u[0];
+        if (r > jc && r < m) P[phys[q] + (int64_t)jc * ld] = l;
+#pragma unroll
+        for (int k = 0; k + 1 < kClSub; ++k) x[q][k] = fma(-l, u[k + 1], x[q][k + 1]);
+      }
+      search(jc + 1);
+    }
+    if (cta == 0 && tid < MAX_PANEL_W) s.phys[tid] = phys[0];
+    // the stores are visible to the rows' later owners
+    if (nctas > 1) cl_sync();
+    else __syncthreads();
+  }
+  // the moves: the W rows of the block in order, then every other row that changed place
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = rbase + kClThreads * q;
+    if (r >= m) continue;
+    int at = r;
+    if (r >= W) {
+      if (phys[q] == r) continue;
+      at = atomicAdd(mv_count, 1);
+    }
+    mv_dst[at] = (int)row0 + r;
+    mv_src[at] = (int)row0 + phys[q];
+  }
+}
+
+// CTAs and rows per thread of the cluster panel for m <= kClMaxRows rows: one row per thread
+// while 16 CTAs suffice (a second and a fourth row per thread cost 50 and 130 us a panel at
+// 1001 rows, more CTAs 1 to 10 us; the step from one CTA to a cluster costs 65 us, a row
+// more per thread the same)
+inline int cl_shape(int m, int *rpt) {
+  int c = 1, r = 1;
+  while (c * kClThreads * r < m) {
+    if (c < kClMaxCtas) c *= 2;
+    else r *= 2;
+  }
+  *rpt = r;
+  return c;
+}
+
+const void *cl_kernel(int rpt) {
+  return rpt == 1   ? (const void *)lu_cluster_panel_kernel<1>
+         : rpt == 2 ? (const void *)lu_cluster_panel_kernel<2>
+                    : (const void *)lu_cluster_panel_kernel<4>;
+}
+
+int cl_config(int ctas, int rpt, cudaStream_t st, cudaLaunchConfig_t *cfg,
+              cudaLaunchAttribute *attr) {
+  const void *fn = cl_kernel(rpt);
+  if (int rc = mo_smem_attr(fn, (int)sizeof(ClSmem))) return rc;
+  MO_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(ctas);
+  cfg->blockDim = dim3(kClThreads);
+  cfg->dynamicSmemBytes = sizeof(ClSmem);
+  cfg->stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim = {(unsigned)ctas, 1, 1};
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  return MO_OK;
 }
 
 // Apply interchanges rows (r0+s) <-> piv[s] (absolute rows of A), s = 0..ns-1 in order,
@@ -521,13 +934,16 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
   const size_t sz_row = (size_t)2 * nblk * W * sizeof(double), sz_rowj = 2 * W * sizeof(double);
   const size_t inv_bytes = 2 * 128 * 128 * sizeof(double);  // two panels' L11 inverses
   const size_t sz_moves = 2 * (2 * MAX_PANEL_W) * sizeof(int) + 64;
-  const size_t total = inv_bytes + sz_val + sz_row + sz_rowj + sz_idx + 64 + 64 + sz_moves;
+  const size_t sz_ubuf = (size_t)kClL * kClSub * sizeof(double);
+  const size_t total =
+      inv_bytes + sz_ubuf + sz_val + sz_row + sz_rowj + sz_idx + 64 + 64 + sz_moves;
   char *ws = nullptr;
   int rc = workspace(ctx, total, (void **)&ws);
   if (rc) return rc;
   double *inv = (double *)ws, *inv_b = inv + 128 * 128;
   PanelScratch sc;
-  char *q = ws + inv_bytes;
+  double *ubuf = (double *)(ws + inv_bytes);
+  char *q = ws + inv_bytes + sz_ubuf;
   sc.cand_val = (double *)q;
   q += sz_val;
   sc.cand_row = (double *)q;
@@ -544,8 +960,39 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
   q += 32;
   int *mv_dst = (int *)q, *mv_src = mv_dst + 2 * MAX_PANEL_W, *mv_count = mv_src + 2 * MAX_PANEL_W;
 
-  // one panel: factor A[k:m, k:k+b], then apply its interchanges left and right of it
+  // rows up to which a panel may run in one cluster (the 16-CTA cluster is not portable: ask)
+  int cl_rows = kClThreads * 8 * 4;
+  if (m > cl_rows) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    int clusters = 0;
+    if ((rc = cl_config(kClMaxCtas, 4, ctx->stream, &cfg, &attr))) return rc;
+    if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(4), &cfg) == cudaSuccess &&
+        clusters > 0)
+      cl_rows = kClMaxRows;
+    else
+      cudaGetLastError();
+  }
+  // one panel: factor A[k:m, k:k+b], then apply its interchanges to the other columns
   auto panel = [&](int k, int b) -> int {
+    if (m - k <= cl_rows) {
+      int rpt;
+      const int ctas = cl_shape(m - k, &rpt);
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr;
+      int r2 = cl_config(ctas, rpt, ctx->stream, &cfg, &attr);
+      if (r2) return r2;
+      ProfScope ps;
+      prof_begin(ctx, ps, MO_PROF_PANEL);
+      double *Pd = A.at(k, k);
+      int64_t pld = A.ld, *pv = piv + k, row0 = k;
+      int pm = m - k, pw = b;
+      void *args[] = {&Pd, &pld, &pm, &pw, &pv, &row0, &ubuf, &mv_dst, &mv_src, &mv_count, &status};
+      const cudaError_t e = cudaLaunchKernelExC(&cfg, cl_kernel(rpt), args);
+      prof_end(ctx, ps, (double)(m - k) * b * b - (double)b * b * b / 3.0, 16.0 * (m - k) * b);
+      MO_CUDA_TRY(e);
+      return laswp_moves(ctx, A, 0, n, mv_dst, mv_src, mv_count, 2 * b);
+    }
     MO_CUDA_TRY(cudaMemsetAsync(sc.barrier, 0, 32, ctx->stream));  // barrier + abort flag
     View Pv = A.sub(k, k, m - k, b);
     const int pm = m - k;
