@@ -119,5 +119,12 @@ def lib() -> ctypes.CDLL:
         fn.restype = i
     L.mo_strerror.argtypes = [i]
     L.mo_strerror.restype = ctypes.c_char_p
+    from . import _tensors
+    _tensors.bind(address(L.mo_set_stream))
     _lib = L
     return L
+
+
+def address(fn) -> int:
+    """the entry point's address, for the extension's direct calls"""
+    return ctypes.cast(fn, ctypes.c_void_p).value

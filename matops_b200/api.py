@@ -16,7 +16,7 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _lib, _tensors
 
 # flags, calgo/cmops.go:19-31
 TRANSA, TRANSB, LOWER, UPPER, LEFT, RIGHT, UNIT, TRANS = 0x1, 0x2, 0x4, 0x8, 0x10, 0x20, 0x40, 0x80
@@ -78,6 +78,23 @@ def context(device: int | None = None) -> ctypes.c_void_p:
     return c
 
 
+_handles: dict[int, int] = {}  # the contexts' addresses
+_entry: dict[str, int] = {}    # addresses of the C functions called through _tensors
+
+
+def _call(form, name, *args):
+    """The C function `name` on the current device's context and stream, its tensors made
+    views in native code (_tensors.call3 / call2 / call2a by signature)."""
+    fn = _entry.get(name)
+    if fn is None:
+        fn = _entry[name] = _lib.address(getattr(_lib.lib(), name))
+    dev = torch.cuda.current_device()
+    ctx = _handles.get(dev)
+    if ctx is None:
+        ctx = _handles[dev] = context(dev).value
+    return form(fn, ctx, torch._C._cuda_getCurrentRawStream(dev), *args)
+
+
 def view(t: torch.Tensor) -> _lib.MoMatrix:
     """mo_matrix of a column-major CUDA float64 tensor view."""
     if t.dim() != 2 or t.dtype != torch.float64 or not t.is_cuda:
@@ -119,17 +136,17 @@ def _err(rc: int, use_on_error: bool = False):
 
 def Mult(C, A, B, alpha: float, beta: float, flags: int = NOTRANS):
     """mmult.go:198 -- C = beta*C + alpha*op(A)*op(B)."""
-    return _err(_lib.lib().mo_mult(context(), view(C), view(A), view(B), alpha, beta, flags))
+    return _err(_call(_tensors.call3, "mo_mult", C, A, B, alpha, beta, flags))
 
 
 def RankUpdateSym(C, A, alpha: float, beta: float, flags: int):
     """mmult.go:426 -- triangle(C) = beta*C + alpha*A*A^T (or A^T*A with TRANSA)."""
-    return _err(_lib.lib().mo_rank_update_sym(context(), view(C), view(A), alpha, beta, flags), True)
+    return _err(_call(_tensors.call2, "mo_rank_update_sym", C, A, alpha, beta, flags), True)
 
 
 def SolveTrm(B, A, alpha: float, flags: int):
     """mmult.go:388 -- B = alpha*op(A)^-1*B (LEFT) or alpha*B*op(A)^-1 (RIGHT)."""
-    return _err(_lib.lib().mo_solve_trm(context(), view(B), view(A), alpha, flags), True)
+    return _err(_call(_tensors.call2a, "mo_solve_trm", B, A, alpha, flags), True)
 
 
 def MultSym(C, A, B, alpha: float, beta: float, flags: int):
@@ -464,8 +481,7 @@ BATCH_MAX_N, BATCH_BUCKETS = 512, 4
 class BatchPlan:
     """A reusable plan (mo_batch) for factoring, and optionally solving, many small
     systems of the given orders in one CUDA-graph launch.  run() takes lists of column-major
-    CUDA float64 matrices (views allowed); their pointer arrays are cached on the device
-    while the same list objects are passed again."""
+    CUDA float64 matrices (views allowed)."""
 
     def __init__(self, kind: int, orders, nrhs: int = 0):
         import numpy as np
@@ -477,8 +493,8 @@ class BatchPlan:
                                         ctypes.byref(self._h))
         if rc:
             raise MatopsError(rc, _lib.lib().mo_strerror(rc).decode())
-        self._arrays = None
-        self._key = None
+        self._host = np.zeros(5 * len(self.orders), dtype=np.int64)  # the table (see run)
+        self._table = self._info = self._given = None
 
     def close(self):
         if self._h:
@@ -491,48 +507,42 @@ class BatchPlan:
         except Exception:
             pass
 
-    def _pack(self, As, Bs, pivs):
-        key = (tuple(a.data_ptr() for a in As), tuple(b.data_ptr() for b in Bs) if Bs else None,
-               tuple(p.data_ptr() for p in pivs) if pivs else None)
-        if key == self._key:
-            return self._arrays
-        dev = As[0].device if As else torch.device("cuda", torch.cuda.current_device())
-
-        def ptrs(ts):
-            return torch.tensor([t.data_ptr() for t in ts], dtype=torch.int64, device=dev)
-
-        def lds(ts):
-            return torch.tensor([view(t).ld for t in ts], dtype=torch.int64, device=dev)
-        for a, n in zip(As, self.orders):
-            if tuple(a.shape) != (int(n), int(n)):
-                raise ValueError("matrix shape does not match the plan's order")
-        arr = {"A": ptrs(As), "lda": lds(As),
-               "B": ptrs(Bs) if Bs else None, "ldb": lds(Bs) if Bs else None,
-               "piv": ptrs(pivs) if pivs else None,
-               "info": torch.zeros(len(As), dtype=torch.int32, device=dev)}
-        self._arrays, self._key = arr, key
-        return arr
-
     def run(self, As, Bs=None, pivs=None):
         """Factor every A (and solve A X = B in place when Bs is given).  pivs: list of CUDA
-        int64 tensors (LU).  Returns the device int32 info tensor (0 = success)."""
-        if len(As) != len(self.orders):
-            raise ValueError("number of matrices does not match the plan")
-        for a in As:
-            view(a)
-        if Bs is not None:
-            for b, n in zip(Bs, self.orders):
-                if view(b).rows != n or b.shape[1] != self.nrhs:
-                    raise ValueError("right-hand side shape does not match the plan")
-        arr = self._pack(As, Bs, pivs)
+        int64 tensors (LU).  Returns the device int32 info tensor (0 = success).
 
-        def p(t):
-            return ctypes.c_void_p(t.data_ptr()) if t is not None else None
-        rc = _lib.lib().mo_batch_run(self._h, p(arr["A"]), p(arr["lda"]), p(arr["B"]),
-                                     p(arr["ldb"]), p(arr["piv"]), p(arr["info"]))
+        The table of addresses and leading dimensions is made anew on every call and goes to
+        the device when it differs from the one that is there."""
+        count = len(self.orders)
+        if len(As) != count:
+            raise ValueError("number of matrices does not match the plan")
+        given = (bool(Bs), bool(pivs))
+        changed = _tensors.batch_pack(As, Bs if given[0] else None, pivs if given[1] else None,
+                                      self.orders.ctypes.data, count, self.nrhs,
+                                      self._host.ctypes.data)
+        if changed or self._given != given or self._table is None:
+            dev = As[0].device if count else torch.device("cuda", torch.cuda.current_device())
+            self._table = None
+            staged = torch.empty(5 * count, dtype=torch.int64, pin_memory=count > 0)
+            staged.numpy()[:] = self._host
+            self._table = staged.to(dev, non_blocking=True)
+            self._info = torch.zeros(count, dtype=torch.int32, device=dev)
+            self._given = given
+            self._stream = torch.cuda.current_stream(dev).cuda_stream
+        here = torch.cuda.current_stream(self._table.device)
+        if here.cuda_stream != self._stream:  # not the stream the memory belongs to
+            self._table.record_stream(here)
+            self._info.record_stream(here)
+        base = self._table.data_ptr()
+
+        def p(k, on=True):
+            return ctypes.c_void_p(base + 8 * k * count) if on else None
+        context()
+        rc = _lib.lib().mo_batch_run(self._h, p(0), p(1), p(2, given[0]), p(3, given[0]),
+                                     p(4, given[1]), ctypes.c_void_p(self._info.data_ptr()))
         if rc:
             raise MatopsError(rc, _lib.lib().mo_strerror(rc).decode())
-        return arr["info"]
+        return self._info
 
     def tune(self, reps: int = 3):
         """Autotune the per-bucket kernel configuration; returns {bucket: [ms cfg0, ms cfg1]}."""
@@ -561,9 +571,12 @@ def DecomposeCHOLAdjoint(L, Lbar, flags: int = LOWER):
 
 def DecomposeCHOLAdjointBatched(Ls, Lbars, flags: int = LOWER):
     """DecomposeCHOLAdjoint for lists of independent matrices (one call, a pool of streams)."""
-    n = len(Ls)
-    arrL = (_lib.MoMatrix * max(n, 1))(*[view(t) for t in Ls])
-    arrG = (_lib.MoMatrix * max(n, 1))(*[view(t) for t in Lbars])
+    n, Lbars = len(Ls), list(Lbars)
+    if len(Lbars) > max(n, 1):
+        raise IndexError("more adjoints than factors")
+    arrL, arrG = (_lib.MoMatrix * max(n, 1))(), (_lib.MoMatrix * max(n, 1))()
+    _tensors.views(Ls, ctypes.addressof(arrL))
+    _tensors.views(Lbars, ctypes.addressof(arrG))
     return _err(_lib.lib().mo_decompose_chol_adjoint_batched(context(), n, arrL, arrG, flags))
 
 

@@ -1,4 +1,5 @@
-"""Build the sm_100a shared library libmatops_b200.so in-tree (nvcc, no GPU needed)."""
+"""Build the sm_100a shared library libmatops_b200.so (nvcc, no GPU needed) and the Python
+extension _tensors.so (g++, torch headers) in-tree."""
 from __future__ import annotations
 
 import glob
@@ -9,6 +10,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmatops_b200.so")
+EXT = os.path.join(HERE, "_tensors.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -29,6 +31,20 @@ def _stale(out: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _ext_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    lib = os.path.join(root, "lib")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[f for d in inc for f in ("-isystem", d)], os.path.join(CSRC, "tensors.cpp"), "-o", EXT,
+            f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
 def build(verbose: bool = False, jobs: int = 8) -> str:
     """Compile every csrc/*.cu to an object (in parallel) and link the shared library."""
     objdir = os.path.join(HERE, "_build")
@@ -36,6 +52,9 @@ def build(verbose: bool = False, jobs: int = 8) -> str:
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(
         os.path.join(HERE, "..", "include", "*.h"))
     procs, objs = [], []
+    if _stale(EXT, [os.path.join(CSRC, "tensors.cpp")] + headers):
+        procs.append(("tensors.cpp", subprocess.Popen(_ext_command(), stdout=subprocess.PIPE,
+                                                      stderr=subprocess.STDOUT)))
     for src in sources():
         obj = os.path.join(objdir, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
@@ -49,7 +68,7 @@ def build(verbose: bool = False, jobs: int = 8) -> str:
     for src, p in procs:
         out, _ = p.communicate()
         if p.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src}:\n{out.decode()}")
+            raise RuntimeError(f"the compiler failed on {src}:\n{out.decode()}")
         if verbose and out:
             print(out.decode(), file=sys.stderr)
     if _stale(LIB, objs):
