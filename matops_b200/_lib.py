@@ -119,10 +119,25 @@ def lib() -> ctypes.CDLL:
         fn.restype = i
     L.mo_strerror.argtypes = [i]
     L.mo_strerror.restype = ctypes.c_char_p
-    from . import _tensors
-    _tensors.bind(address(L.mo_set_stream))
+    ext().bind(address(L.mo_set_stream))
     _lib = L
     return L
+
+
+_ext = None
+
+
+def ext():
+    """the _tensors extension (built like the library; no fallback either)"""
+    global _ext
+    if _ext is None:
+        try:
+            from . import _tensors
+        except ImportError as e:
+            raise ImportError("the _tensors extension is missing: build it with "
+                              "`python -m matops_b200.build` (there is no fallback)") from e
+        _ext = _tensors
+    return _ext
 
 
 def address(fn) -> int:

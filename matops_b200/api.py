@@ -16,7 +16,7 @@ import ctypes
 
 import torch
 
-from . import _lib, _tensors
+from . import _lib
 
 # flags, calgo/cmops.go:19-31
 TRANSA, TRANSB, LOWER, UPPER, LEFT, RIGHT, UNIT, TRANS = 0x1, 0x2, 0x4, 0x8, 0x10, 0x20, 0x40, 0x80
@@ -79,20 +79,21 @@ def context(device: int | None = None) -> ctypes.c_void_p:
 
 
 _handles: dict[int, int] = {}  # the contexts' addresses
-_entry: dict[str, int] = {}    # addresses of the C functions called through _tensors
+_entry: dict[str, tuple] = {}  # (extension function, C function's address) by C name
 
 
 def _call(form, name, *args):
     """The C function `name` on the current device's context and stream, its tensors made
-    views in native code (_tensors.call3 / call2 / call2a by signature)."""
-    fn = _entry.get(name)
-    if fn is None:
-        fn = _entry[name] = _lib.address(getattr(_lib.lib(), name))
+    views in native code (the extension's call3 / call2 / call2a by signature)."""
+    entry = _entry.get(name)
+    if entry is None:
+        lib = _lib.lib()
+        entry = _entry[name] = (getattr(_lib.ext(), form), _lib.address(getattr(lib, name)))
     dev = torch.cuda.current_device()
     ctx = _handles.get(dev)
     if ctx is None:
         ctx = _handles[dev] = context(dev).value
-    return form(fn, ctx, torch._C._cuda_getCurrentRawStream(dev), *args)
+    return entry[0](entry[1], ctx, torch._C._cuda_getCurrentRawStream(dev), *args)
 
 
 def view(t: torch.Tensor) -> _lib.MoMatrix:
@@ -136,17 +137,17 @@ def _err(rc: int, use_on_error: bool = False):
 
 def Mult(C, A, B, alpha: float, beta: float, flags: int = NOTRANS):
     """mmult.go:198 -- C = beta*C + alpha*op(A)*op(B)."""
-    return _err(_call(_tensors.call3, "mo_mult", C, A, B, alpha, beta, flags))
+    return _err(_call("call3", "mo_mult", C, A, B, alpha, beta, flags))
 
 
 def RankUpdateSym(C, A, alpha: float, beta: float, flags: int):
     """mmult.go:426 -- triangle(C) = beta*C + alpha*A*A^T (or A^T*A with TRANSA)."""
-    return _err(_call(_tensors.call2, "mo_rank_update_sym", C, A, alpha, beta, flags), True)
+    return _err(_call("call2", "mo_rank_update_sym", C, A, alpha, beta, flags), True)
 
 
 def SolveTrm(B, A, alpha: float, flags: int):
     """mmult.go:388 -- B = alpha*op(A)^-1*B (LEFT) or alpha*B*op(A)^-1 (RIGHT)."""
-    return _err(_call(_tensors.call2a, "mo_solve_trm", B, A, alpha, flags), True)
+    return _err(_call("call2a", "mo_solve_trm", B, A, alpha, flags), True)
 
 
 def MultSym(C, A, B, alpha: float, beta: float, flags: int):
@@ -517,7 +518,7 @@ class BatchPlan:
         if len(As) != count:
             raise ValueError("number of matrices does not match the plan")
         given = (bool(Bs), bool(pivs))
-        changed = _tensors.batch_pack(As, Bs if given[0] else None, pivs if given[1] else None,
+        changed = _lib.ext().batch_pack(As, Bs if given[0] else None, pivs if given[1] else None,
                                       self.orders.ctypes.data, count, self.nrhs,
                                       self._host.ctypes.data)
         if changed or self._given != given or self._table is None:
@@ -575,8 +576,8 @@ def DecomposeCHOLAdjointBatched(Ls, Lbars, flags: int = LOWER):
     if len(Lbars) > max(n, 1):
         raise IndexError("more adjoints than factors")
     arrL, arrG = (_lib.MoMatrix * max(n, 1))(), (_lib.MoMatrix * max(n, 1))()
-    _tensors.views(Ls, ctypes.addressof(arrL))
-    _tensors.views(Lbars, ctypes.addressof(arrG))
+    _lib.ext().views(Ls, ctypes.addressof(arrL))
+    _lib.ext().views(Lbars, ctypes.addressof(arrG))
     return _err(_lib.lib().mo_decompose_chol_adjoint_batched(context(), n, arrL, arrG, flags))
 
 
