@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm.cuh"
@@ -544,6 +545,117 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
+// ---- few small tiles -------------------------------------------------------------------
+// A product with a short K whose 128 x 64 tiles would occupy a fraction of the SMs (a panel
+// of a factorization, a small user matrix) runs on 32 x 32 tiles instead, one CTA of four
+// warps each: four to eight times the CTAs, no tensor maps, and little padding.  In-place
+// products keep one CTA per strip that is both read and written: 32 x 128 tiles where C is
+// op(A) (N <= 128), 128 x 32 where C is op(B) (M <= 128).  Operands of any alignment come by
+// 8-byte cp.async into a ring of 16-wide slabs, k-row by k-row with a row stride of 4 mod 16
+// doubles, so the fragment loads touch every bank once.
+template <int TM, int TN>
+struct SmallGeo {
+  static constexpr int STAGES = TM * TN > 2048 ? 4 : 6;
+  static constexpr int LA = TM + 4, LBS = TN + 4;
+  static constexpr int STAGE = 16 * (LA + LBS);
+  static constexpr int SMEM = STAGES * STAGE * 8;
+};
+
+template <bool A_KMAJ, bool B_KMAJ, int TM, int TN, int WM, int WN>
+__global__ void __launch_bounds__(WM *WN * 32) dgemm_small_kernel(const KParams p) {
+  using G = SmallGeo<TM, TN>;
+  constexpr int NT = WM * WN * 32, FM = TM / WM / 16, FN = TN / WN / 8, STG = G::STAGES;
+  extern __shared__ double small_smem[];
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  if ((p.mode == kSyrkLower || p.mode == kGemmLower) && m0 + TM - 1 < n0) return;
+  if ((p.mode == kSyrkUpper || p.mode == kGemmUpper) && m0 > n0 + TN - 1) return;
+  if (p.skip && *(volatile const int *)p.skip) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int wr = (warp % WM) * (TM / WM), wc = (warp / WM) * (TN / WN);
+
+  // one operand's slab: ROWS x 16 at s[k * ld + mn]
+  auto fetch = [&](auto kmaj, auto rows, double *s, int ls, const double *src, int64_t ld, int mn0,
+                   int MN, int k0) {
+    constexpr bool KM = decltype(kmaj)::value;
+    constexpr int ROWS = decltype(rows)::value;
+#pragma unroll
+    for (int e = tid; e < ROWS * 16; e += NT) {
+      const int k = KM ? e & 15 : e / ROWS, mn = KM ? e >> 4 : e % ROWS;
+      const bool ok = mn0 + mn < MN && k0 + k < p.K;
+      const double *q = KM ? src + (k0 + k) + (int64_t)(mn0 + mn) * ld
+                           : src + (mn0 + mn) + (int64_t)(k0 + k) * ld;
+      cp_async_8(s + k * ls + mn, ok ? q : src, ok ? 8u : 0u);
+    }
+  };
+  auto load = [&](int kt) {
+    if (kt < p.kt) {
+      double *s = small_smem + (kt % STG) * G::STAGE;
+      fetch(std::integral_constant<bool, A_KMAJ>{}, std::integral_constant<int, TM>{}, s, G::LA, p.A,
+            p.lda, m0, p.M, kt * BK);
+      fetch(std::integral_constant<bool, B_KMAJ>{}, std::integral_constant<int, TN>{},
+            s + 16 * G::LA, G::LBS, p.B, p.ldb, n0, p.N, kt * BK);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[FM][FN][4] = {};
+#pragma unroll
+  for (int s = 0; s < STG - 1; ++s) load(s);
+  for (int kt = 0; kt < p.kt; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STG - 2) : "memory");
+    __syncthreads();
+    load(kt + STG - 1);
+    const double *sa = small_smem + (kt % STG) * G::STAGE + t * G::LA + wr + g;
+    const double *sb = small_smem + (kt % STG) * G::STAGE + 16 * G::LA + t * G::LBS + wc + g;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      double a[FM][2], b[FN];
+#pragma unroll
+      for (int i = 0; i < FM; ++i) {
+        a[i][0] = sa[4 * q * G::LA + 16 * i];
+        a[i][1] = sa[4 * q * G::LA + 16 * i + 8];
+      }
+#pragma unroll
+      for (int j = 0; j < FN; ++j) b[j] = sb[4 * q * G::LBS + 8 * j];
+#pragma unroll
+      for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j) dmma_16x8x4(acc[i][j], a[i][0], a[i][1], b[j]);
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  // epilogue, as the engine's general one: every C is read before any is written
+  const bool need_c = p.beta != 0.0 || p.beta_block > 0;
+#pragma unroll
+  for (int i = 0; i < FM; ++i) {
+    double cv[FN][4];
+    unsigned keep = 0;
+#pragma unroll
+    for (int j = 0; j < FN; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = m0 + wr + 16 * i + g + 8 * (r >> 1), col = n0 + wc + 8 * j + 2 * t + (r & 1);
+        bool k = row < p.M && col < p.N;
+        if ((p.mode == kSyrkLower || p.mode == kGemmLower) && row < col) k = false;
+        if ((p.mode == kSyrkUpper || p.mode == kGemmUpper) && row > col) k = false;
+        keep |= (k ? 1u : 0u) << (4 * j + r);
+        cv[j][r] = (k && need_c) ? __ldcg(p.C + row + (int64_t)col * p.ldc) : 0.0;
+      }
+#pragma unroll
+    for (int j = 0; j < FN; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (!(keep >> (4 * j + r) & 1u)) continue;
+        const int row = m0 + wr + 16 * i + g + 8 * (r >> 1), col = n0 + wc + 8 * j + 2 * t + (r & 1);
+        double bet = p.beta;
+        if (p.beta_block > 0 && (row / p.beta_block) != (col / p.beta_block)) bet = 1.0;
+        double v = p.alpha * acc[i][j][r];
+        if (bet != 0.0) v = fma(bet, cv[j][r], v);
+        p.C[row + (int64_t)col * p.ldc] = v;
+      }
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
@@ -607,6 +719,23 @@ int dispatch(bool ak, bool bk, const KParams &kp, const CUtensorMap &ta, const C
             : launch_inst<false, false, TMA, WIDE>(kp, ta, tb, grid, st);
 }
 
+template <int TM, int TN, int WM, int WN>
+int launch_small(bool ak, bool bk, const KParams &kp, cudaStream_t st) {
+  constexpr int SMEM = SmallGeo<TM, TN>::SMEM;
+  const dim3 grid((kp.M + TM - 1) / TM, (kp.N + TN - 1) / TN);
+  auto go = [&](auto kern) -> int {
+    if (SMEM > 48 * 1024)
+      if (int rc = mo_smem_attr((const void *)kern, SMEM)) return rc;
+    kern<<<grid, WM * WN * 32, SMEM, st>>>(kp);
+    MO_CUDA_TRY(cudaGetLastError());
+    return MO_OK;
+  };
+  if (ak) return bk ? go(dgemm_small_kernel<true, true, TM, TN, WM, WN>)
+                    : go(dgemm_small_kernel<true, false, TM, TN, WM, WN>);
+  return bk ? go(dgemm_small_kernel<false, true, TM, TN, WM, WN>)
+            : go(dgemm_small_kernel<false, false, TM, TN, WM, WN>);
+}
+
 }  // namespace
 
 bool gemm_tma_ok(const GemmArgs &a) {
@@ -615,6 +744,17 @@ bool gemm_tma_ok(const GemmArgs &a) {
 }
 
 size_t gemm_partial_bytes(int sms) { return 2 * (size_t)sms * TILE_DBL * sizeof(double); }
+
+// Whether a product goes to the small-tile kernel: up to 2^27 multiply-adds, where the engine's
+// start (barriers, tensor maps, the first slabs) and its large tiles on a few SMs cost more
+// than the small tiles' extra operand traffic.  Measured, engine / small tiles in us: 64^3
+// 12.3 / 4.1, 512 x 128 x 128 18.4 / 6.2, 1000 x 1000 x 128 24.6 / 19.3, 500^3 32.8 / 18.4; above,
+// 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  A K past 4096 on few tiles is the engine's,
+// which splits it (128 x 128 x 4000: 119 / 82 us).
+static bool small_product(const GemmArgs &a) {
+  const double tri = a.mode == kSyrkLower || a.mode == kSyrkUpper ? 0.5 : 1.0;
+  return a.K <= 4096 && a.N <= 65535 * 32 && tri * a.M * (double)a.N * a.K <= 134217728.0;
+}
 
 int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0) return MO_OK;
@@ -656,6 +796,13 @@ int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
   kp.kt = (kp.K + BK - 1) / BK;
   int sms = a.sms > 0 ? a.sms : 148;
   if (a.max_ctas > 0 && a.max_ctas < sms) sms = a.max_ctas;
+  // few tiles: 32 x 32 ones (or strips, in place)
+  if (!a.force_fallback && small_product(a)) {
+    const bool ak = a.transA, bk = !a.transB;
+    if (a.C == a.A) return launch_small<32, 128, 2, 4>(ak, bk, kp, stream);
+    if (a.C == a.B) return launch_small<128, 32, 4, 2>(ak, bk, kp, stream);
+    return launch_small<32, 32, 2, 2>(ak, bk, kp, stream);
+  }
   // Schedule: whole tiles round-robin over the workers (two per CTA) of a persistent grid;
   // when a GEMM has only a few, unequal waves (e.g. 512 tiles on 2 x 148 workers), the last
   // one or two waves are split along K evenly over all workers (stream-K) and finished by

@@ -1,5 +1,6 @@
-"""The DMMA engine's tile edges: 128 x 64 and 64 x 128 tiles, k-slabs of 16, operands by TMA
-(even leading dimensions) and by cp.async (odd ones), and in-place products, against numpy.
+"""Mult's tile edges: the engine's 128 x 64 and 64 x 128 tiles with operands by TMA (even leading
+dimensions) and by cp.async (odd ones), the 32 x 32 tiles and strips of products up to 2^27
+multiply-adds, k-slabs of 16, and in-place products, against numpy.
 Bound: 4 k eps (|alpha| ||A|| ||B|| + |beta| ||C||), as in the parity tests of Mult."""
 import numpy as np
 import pytest
@@ -22,7 +23,8 @@ def _dev(gpu, a, ld):
 @pytest.mark.parametrize("flags", [0, TA, TB, TA | TB])
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 129, 15), (64, 65, 16), (65, 64, 17), (64, 128, 33),
                                    (127, 63, 31), (128, 64, 48), (129, 65, 64), (257, 191, 79),
-                                   (33, 400, 130), (640, 1088, 208), (2049, 65, 1040),
+                                   (33, 400, 130), (31, 33, 4096), (32, 65, 4097),
+                                   (2300, 456, 129), (640, 1088, 208), (2049, 65, 1040),
                                    (2560, 2432, 40)])
 def test_tile_edges(gpu, rng, m, n, k, flags, odd):
     A = rng.uniform(-1, 1, (k, m) if flags & TA else (m, k))
@@ -59,7 +61,8 @@ def test_triangle_tiles(gpu, rng, n, k, flags):
 
 
 @pytest.mark.parametrize("side", [0x10, 0x20])
-@pytest.mark.parametrize("n,nrhs", [(100, 200), (128, 130), (129, 65), (300, 257)])
+@pytest.mark.parametrize("n,nrhs", [(100, 200), (128, 130), (129, 65), (300, 257), (31, 97),
+                                    (160, 9001)])
 def test_in_place_products(gpu, rng, n, nrhs, side):
     """SolveTrm above 64 right-hand sides multiplies by block inverses in place, from the left
     (C = op(B)) and from the right (C = op(A)); odd orders take the cp.async producer.  Bound:
