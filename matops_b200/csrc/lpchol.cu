@@ -28,69 +28,35 @@ namespace {
 
 constexpr int NB = 128;
 
-// shared memory of lp_diag_kernel: the FP32 block plus the inverse's scratch sub-blocks
-constexpr int LP_DIAG_SMEM = (TRI_MAX * LDS + 4 * SUB * (SUB + 1)) * (int)sizeof(float);
-
-// W block (FP32, column-major) -> S (FP32 lower, row-major, LDS)
-__device__ inline void lp_load_block(float *S, const float *G, int64_t ld) {
-  for (int base = threadIdx.x; base < NB * NB; base += 8 * blockDim.x) {
-    float v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = base + u * blockDim.x;
-      const int i = e % NB, j = e / NB;
-      v[u] = (e < NB * NB && i >= j) ? G[i + (int64_t)j * ld] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = base + u * blockDim.x;
-      if (e < NB * NB) S[(e % NB) * LDS + e / NB] = v[u];
-    }
-  }
-}
-
-// The diagonal block is factored and inverted in FP32, the precision of the working
-// matrix it comes from and goes back to: its rounding is below that of the split-product
-// updates that formed it (BF16x3) or equal to it (TF32x3), and the FP32 column chain
-// (single-instruction reciprocal square root, 4-cycle FMA, one shuffle per value) is much
-// shorter than the FP64 one.  The inverse goes out as FP64 (for the refinement solves)
-// and split (for the panel product).
+// The diagonal block comes from the FP32 working matrix and is factored and inverted in FP64 (on
+// the FP64 tensor pipe; an FP32 factorization by 32-column leaves took 68 us a block, this
+// one 43); the factor goes back rounded to FP32, the inverse out as FP64 (for the refinement
+// solves) and split (for the panel product).
 template <int PREC>
 __global__ void __launch_bounds__(TRI_THREADS)
     lp_diag_kernel(float *W, int64_t ldw, double *inv, char *ihi, char *ilo, int *info,
                    double *bad_value, int col0, int n_true) {
   if (*(volatile int *)info != 0) return;
-  extern __shared__ float smf[];
-  float *S = smf;
-  float *Wk = smf + TRI_MAX * LDS;
-  __shared__ int s_bad;
-  __shared__ double s_badv;
-  lp_load_block(S, W, ldw);
+  extern __shared__ double smd[];
+  const TriSmem t(smd);
+  tri_load_lower(t.S, W, ldw, NB, false, false);
   __syncthreads();
-  tri_potrf_lower(S, NB, &s_bad, &s_badv);
-  if (s_bad >= 0) {
+  double badv;
+  const int bad = tri_potrf_inverse(t, NB, &badv);
+  if (bad >= 0) {
     // a failure inside the identity padding cannot happen; report the true column
-    if (threadIdx.x == 0 && col0 + s_bad < n_true) {
-      *info = col0 + s_bad + 1;
-      *bad_value = s_badv;
+    if (threadIdx.x == 0 && col0 + bad < n_true) {
+      *info = col0 + bad + 1;
+      *bad_value = badv;
     }
     return;
   }
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int i = e % NB, j = e / NB;
-    if (i >= j) W[i + (int64_t)j * ldw] = S[i * LDS + j];
-  }
-  __syncthreads();
-  tri_inverse_lower(S, NB, Wk);
-  __syncthreads();
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int i = e % NB, j = e / NB;
-    inv[i + j * NB] = (i >= j) ? (double)S[i * LDS + j] : 0.0;
-  }
+  tri_store_lower(t.S, W, ldw, NB, false);
+  tri_store_inverse(t, inv, NB, NB, false);
   // split inverse, K-major: row r = row r of L11^-1 (the B operand of A21 * L11^-T)
   for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
     const int r = e / NB, k = e % NB;
-    const float x = (r >= k) ? S[r * LDS + k] : 0.f;
+    const float x = (float)tri_inv_at(t, r, k);
     if (PREC == kLpBf16x3) {
       const __nv_bfloat16 h = __float2bfloat16_rn(x);
       const __nv_bfloat16 l = __float2bfloat16_rn(x - __bfloat162float(h));
@@ -143,7 +109,7 @@ __global__ void __launch_bounds__(256) lp_convert_kernel(const double *A, int64_
 
 template <int PREC>
 int set_lp_diag_smem() {
-  return mo_smem_attr((const void *)lp_diag_kernel<PREC>, LP_DIAG_SMEM);
+  return mo_smem_attr((const void *)lp_diag_kernel<PREC>, TRI_SMEM_BYTES);
 }
 
 // diagonal block + panel of step k on ctx->stream; P receives the split L21.  The split
@@ -155,10 +121,10 @@ int lp_panel(mo_ctx *ctx, LpChol &f, int k, int *d_info, double *d_bad, const Lp
   ProfScope ps;
   prof_begin(ctx, ps, MO_PROF_DIAG);
   if (f.prec == kLpBf16x3)
-    lp_diag_kernel<kLpBf16x3><<<1, TRI_THREADS, LP_DIAG_SMEM, ctx->stream>>>(
+    lp_diag_kernel<kLpBf16x3><<<1, TRI_THREADS, TRI_SMEM_BYTES, ctx->stream>>>(
         Wkk, f.ldw, inv, (char *)f.Linv.hi, (char *)f.Linv.lo, d_info, d_bad, k, f.n);
   else
-    lp_diag_kernel<kLpTf32x3><<<1, TRI_THREADS, LP_DIAG_SMEM, ctx->stream>>>(
+    lp_diag_kernel<kLpTf32x3><<<1, TRI_THREADS, TRI_SMEM_BYTES, ctx->stream>>>(
         Wkk, f.ldw, inv, (char *)f.Linv.hi, (char *)f.Linv.lo, d_info, d_bad, k, f.n);
   prof_end(ctx, ps, 2.0 * NB * NB * NB / 3.0, 4.0 * 2.0 * NB * NB + 8.0 * NB * NB);
   MO_CUDA_TRY(cudaGetLastError());

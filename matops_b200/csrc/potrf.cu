@@ -20,27 +20,22 @@ __global__ void __launch_bounds__(TRI_THREADS)
                       double *bad_value, int col0) {
   if (*(volatile int *)info != 0) return;  // an earlier block failed
   extern __shared__ double sm[];
-  double *S = sm;
-  double *W = sm + TRI_MAX * LDS;
-  __shared__ int s_bad;
-  __shared__ double s_badv;
+  const TriSmem t(sm);
   const int NP = round_up32(n);
   // upper storage: A = U^T U with U^T lower, so load/store the transpose
-  tri_load_lower(S, A, lda, n, upper, false);
+  tri_load_lower(t.S, A, lda, n, upper, false);
   __syncthreads();
-  tri_potrf_lower(S, NP, &s_bad, &s_badv);
-  if (s_bad >= 0) {
+  double badv;
+  const int bad = tri_potrf_inverse(t, NP, &badv);
+  if (bad >= 0) {
     if (threadIdx.x == 0) {
-      *info = col0 + s_bad + 1;
-      *bad_value = s_badv;
+      *info = col0 + bad + 1;
+      *bad_value = badv;
     }
     return;
   }
-  tri_store_lower(S, A, lda, n, upper, false);
-  __syncthreads();
-  tri_inverse_lower(S, NP, W);
-  __syncthreads();
-  tri_store_lower(S, inv, NB, n, false, true);
+  tri_store_lower(t.S, A, lda, n, upper);
+  tri_store_inverse(t, inv, NB, n, false);
 }
 
 }  // namespace

@@ -21,16 +21,14 @@ __global__ void __launch_bounds__(TRI_THREADS)
     trtri_blocks_kernel(const double *A, int64_t lda, int N, bool load_transposed,
                         bool store_transposed, bool unit, double *inv) {
   extern __shared__ double sm[];
-  double *S = sm;
-  double *W = sm + TRI_MAX * LDS;
+  const TriSmem t(sm);
   const int r0 = blockIdx.x * NBT;
   const int n = min(NBT, N - r0);
   const int NP = round_up32(n);
-  tri_load_lower(S, A + r0 + (int64_t)r0 * lda, lda, n, load_transposed, unit);
+  tri_load_lower(t.S, A + r0 + (int64_t)r0 * lda, lda, n, load_transposed, unit);
   __syncthreads();
-  tri_inverse_lower(S, NP, W);
-  __syncthreads();
-  tri_store_lower(S, inv + (size_t)blockIdx.x * NBT * NBT, NBT, n, store_transposed, true);
+  tri_inverse_lower(t, NP);
+  tri_store_inverse(t, inv + (size_t)blockIdx.x * NBT * NBT, NBT, n, store_transposed);
 }
 
 int set_tri_smem(const void *fn) {
