@@ -588,8 +588,8 @@ __global__ void __launch_bounds__(WM *WN * 32) dgemm_small_kernel(const KParams 
       cp_async_8(s + k * ls + mn, ok ? q : src, ok ? 8u : 0u);
     }
   };
-  auto load = [&](int kt) {
-    if (kt < p.kt) {
+  auto load = [&](int kt, int end) {
+    if (kt < end) {
       double *s = small_smem + (kt % STG) * G::STAGE;
       fetch(std::integral_constant<bool, A_KMAJ>{}, std::integral_constant<int, TM>{}, s, G::LA, p.A,
             p.lda, m0, p.M, kt * BK);
@@ -598,13 +598,15 @@ __global__ void __launch_bounds__(WM *WN * 32) dgemm_small_kernel(const KParams 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  // this CTA's slabs: all of them, or a chunk of K (blockIdx.z) whose sums go to p.partial
+  const int kt0 = blockIdx.z * p.sk_chunk, kt1 = min(p.kt, kt0 + p.sk_chunk);
   double acc[FM][FN][4] = {};
 #pragma unroll
-  for (int s = 0; s < STG - 1; ++s) load(s);
-  for (int kt = 0; kt < p.kt; ++kt) {
+  for (int s = 0; s < STG - 1; ++s) load(kt0 + s, kt1);
+  for (int kt = kt0; kt < kt1; ++kt) {
     asm volatile("cp.async.wait_group %0;" ::"n"(STG - 2) : "memory");
     __syncthreads();
-    load(kt + STG - 1);
+    load(kt + STG - 1, kt1);
     const double *sa = small_smem + (kt % STG) * G::STAGE + t * G::LA + wr + g;
     const double *sb = small_smem + (kt % STG) * G::STAGE + 16 * G::LA + t * G::LBS + wc + g;
 #pragma unroll
@@ -624,6 +626,18 @@ __global__ void __launch_bounds__(WM *WN * 32) dgemm_small_kernel(const KParams 
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  if (gridDim.z > 1) {
+    double *out = p.partial + ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x * (TM * TN) +
+                  (size_t)blockIdx.x * (TM * TN);
+#pragma unroll
+    for (int i = 0; i < FM; ++i)
+#pragma unroll
+      for (int j = 0; j < FN; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          out[(wr + 16 * i + g + 8 * (r >> 1)) + (wc + 8 * j + 2 * t + (r & 1)) * TM] = acc[i][j][r];
+    return;
+  }
   // epilogue, as the engine's general one: every C is read before any is written
   const bool need_c = p.beta != 0.0 || p.beta_block > 0;
 #pragma unroll
@@ -654,6 +668,22 @@ __global__ void __launch_bounds__(WM *WN * 32) dgemm_small_kernel(const KParams 
         p.C[row + (int64_t)col * p.ldc] = v;
       }
   }
+}
+
+// C = alpha * (the K chunks' partial 32 x 32 tiles, added in order) + beta * C
+__global__ void __launch_bounds__(256) small_reduce_kernel(const KParams p, int chunks) {
+  const int tiles_m = (p.M + 31) / 32, tiles = tiles_m * ((p.N + 31) / 32);
+  const int64_t e = blockIdx.x * (int64_t)256 + threadIdx.x;
+  if (e >= (int64_t)p.M * p.N || (p.skip && *(volatile const int *)p.skip)) return;
+  const int row = (int)(e % p.M), col = (int)(e / p.M);
+  const double *src = p.partial + ((size_t)(col >> 5) * tiles_m + (row >> 5)) * 1024 + (row & 31) +
+                      32 * (col & 31);
+  double sum = 0.0;
+#pragma unroll 8
+  for (int c = 0; c < chunks; ++c) sum += __ldcg(src + (size_t)c * tiles * 1024);
+  double *dst = p.C + row + (int64_t)col * p.ldc;
+  const double v = p.alpha * sum;
+  *dst = p.beta != 0.0 ? fma(p.beta, *dst, v) : v;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -720,9 +750,9 @@ int dispatch(bool ak, bool bk, const KParams &kp, const CUtensorMap &ta, const C
 }
 
 template <int TM, int TN, int WM, int WN>
-int launch_small(bool ak, bool bk, const KParams &kp, cudaStream_t st) {
+int launch_small(bool ak, bool bk, const KParams &kp, cudaStream_t st, int chunks = 1) {
   constexpr int SMEM = SmallGeo<TM, TN>::SMEM;
-  const dim3 grid((kp.M + TM - 1) / TM, (kp.N + TN - 1) / TN);
+  const dim3 grid((kp.M + TM - 1) / TM, (kp.N + TN - 1) / TN, chunks);
   auto go = [&](auto kern) -> int {
     if (SMEM > 48 * 1024)
       if (int rc = mo_smem_attr((const void *)kern, SMEM)) return rc;
@@ -745,15 +775,25 @@ bool gemm_tma_ok(const GemmArgs &a) {
 
 size_t gemm_partial_bytes(int sms) { return 2 * (size_t)sms * TILE_DBL * sizeof(double); }
 
-// Whether a product goes to the small-tile kernel: up to 2^27 multiply-adds, where the engine's
-// start (barriers, tensor maps, the first slabs) and its large tiles on a few SMs cost more
-// than the small tiles' extra operand traffic.  Measured, engine / small tiles in us: 64^3
-// 12.3 / 4.1, 512 x 128 x 128 18.4 / 6.2, 1000 x 1000 x 128 24.6 / 19.3, 500^3 32.8 / 18.4; above,
-// 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  A K past 4096 on few tiles is the engine's,
-// which splits it (128 x 128 x 4000: 119 / 82 us).
-static bool small_product(const GemmArgs &a) {
+// Whether a product goes to the small-tile kernel, and in how many chunks of K (0: the engine).
+// Up to 2^27 multiply-adds the engine's start (barriers, tensor maps, the first slabs) and its
+// large tiles on a few SMs cost more than the small tiles' extra operand traffic.  Measured,
+// engine / small tiles in us: 64^3 12.3 / 4.1, 512 x 128 x 128 18.4 / 6.2, 1000 x 1000 x 128 24.6 /
+// 19.3, 500^3 32.8 / 18.4; above, 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  A C of a few
+// small tiles with a long K is split along K, two CTAs per SM with at least 128 rows of K each,
+// and the partial tiles are added in order by a second kernel, up to 2^29
+// multiply-adds: 128 x 128 x 8000 219 / 21, 512 x 128 x 8000 103 / 62, 1000 x 128 x 8000 101 / 119.
+static int small_chunks(const GemmArgs &a, int sms) {
   const double tri = a.mode == kSyrkLower || a.mode == kSyrkUpper ? 0.5 : 1.0;
-  return a.K <= 4096 && a.N <= 65535 * 32 && tri * a.M * (double)a.N * a.K <= 134217728.0;
+  const double work = tri * a.M * (double)a.N * a.K;
+  if (a.force_fallback || a.N > 65535 * 32) return 0;
+  const long long tiles = (long long)((a.M + 31) / 32) * ((a.N + 31) / 32);
+  if (a.mode == kGemm && a.sk_partial && a.C != a.A && a.C != a.B && a.K >= 512 && tiles < sms &&
+      work <= 536870912.0) {
+    const int chunks = (int)std::min<long long>(a.K / 128, 2 * sms / tiles);
+    if (chunks > 1) return chunks;
+  }
+  return a.K <= 4096 && work <= 134217728.0 ? 1 : 0;
 }
 
 int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
@@ -796,12 +836,19 @@ int launch_gemm(const GemmArgs &a, cudaStream_t stream) {
   kp.kt = (kp.K + BK - 1) / BK;
   int sms = a.sms > 0 ? a.sms : 148;
   if (a.max_ctas > 0 && a.max_ctas < sms) sms = a.max_ctas;
-  // few tiles: 32 x 32 ones (or strips, in place)
-  if (!a.force_fallback && small_product(a)) {
+  // few tiles: 32 x 32 ones (or strips, in place), perhaps in chunks of K
+  if (int chunks = small_chunks(a, sms)) {
     const bool ak = a.transA, bk = !a.transB;
+    kp.sk_chunk = (kp.kt + chunks - 1) / chunks;
     if (a.C == a.A) return launch_small<32, 128, 2, 4>(ak, bk, kp, stream);
     if (a.C == a.B) return launch_small<128, 32, 4, 2>(ak, bk, kp, stream);
-    return launch_small<32, 32, 2, 2>(ak, bk, kp, stream);
+    kp.partial = a.sk_partial;
+    chunks = kp.sk_chunk > 0 ? (kp.kt + kp.sk_chunk - 1) / kp.sk_chunk : 1;
+    const int rc = launch_small<32, 32, 2, 2>(ak, bk, kp, stream, chunks);
+    if (rc || chunks == 1) return rc;
+    small_reduce_kernel<<<(unsigned)(((int64_t)a.M * a.N + 255) / 256), 256, 0, stream>>>(kp, chunks);
+    MO_CUDA_TRY(cudaGetLastError());
+    return MO_OK;
   }
   // Schedule: whole tiles round-robin over the workers (two per CTA) of a persistent grid;
   // when a GEMM has only a few, unequal waves (e.g. 512 tiles on 2 x 148 workers), the last

@@ -18,6 +18,7 @@
 #include <climits>
 #include <utility>
 
+#include "cluster.cuh"
 #include "context.cuh"
 #include "tri.cuh"
 
@@ -290,39 +291,6 @@ struct ClSmem {
   __align__(16) double L[(kClL + 1) * kClLd];  // (CTA 0) finished rows of L, transposed
 };
 
-__device__ __forceinline__ uint32_t cl_map(const void *p, int cta) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cta));
-  return a;
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-                   : "memory");
-}
-// `src` (this CTA's shared memory) to the same place `dst` of every CTA of the cluster, the
-// bytes counted on that CTA's barrier `bar`: the calling warp's lane pair (2 c, 2 c + 1)
-// writes CTA c's copy, nine 16-byte pieces in all.  (Plain remote stores need a cluster
-// barrier with release semantics, which also waits for the multipliers' global stores: 1330
-// cycles a column.)
-__device__ __forceinline__ void cl_send(ClRow *dst, const ClRow *src, uint64_t *bar, int lane,
-                                        int nctas) {
-  const int c = lane >> 1;
-  if (c >= nctas) return;
-  const uint32_t to = cl_map(dst, c), mb = cl_map(bar, c);
-  const double2 *s = reinterpret_cast<const double2 *>(src);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    const int p = 2 * i + (lane & 1);
-    if (p < 9) {
-      const double2 v = s[p];
-      asm volatile(
-          "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
-              to + 16 * p),
-          "d"(v.x), "d"(v.y), "r"(mb)
-          : "memory");
-    }
-  }
-}
 static_assert(sizeof(ClRow) == 9 * 16, "row packet");
 static_assert(kClThreads == kClSub * kClSub && kClThreads >= MAX_PANEL_W, "index splits below");
 
@@ -521,7 +489,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
           to.phys = phys[0];
         }
         __syncwarp();
-        if (nctas > 1) cl_send(&s.rowj[par], &s.ownj, &s.bar[par], lane, nctas);
+        if (nctas > 1) cl_send<9>(&s.rowj[par], &s.ownj, &s.bar[par], lane, nctas);
       }
       __syncthreads();
       hi = s.red_hi[par][lane & (kClWarps - 1)];
@@ -546,7 +514,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
             to.phys = phys[q];
           }
         __syncwarp();
-        if (nctas > 1) cl_send(&s.recv[par][cta], &s.own, &s.bar[par], lane, nctas);
+        if (nctas > 1) cl_send<9>(&s.recv[par][cta], &s.own, &s.bar[par], lane, nctas);
       }
       // every warp picks the pivot: largest key, lowest row
       if (nctas > 1) {

@@ -9,8 +9,9 @@
 // 121-129, 433-453).  A holds R on and above its diagonal and the reflectors below it.
 //
 // Device form, per 128-column block of A:
-//   * four 32-column panels, each factored by ONE cooperative kernel: every CTA keeps a
-//     slice of the panel's rows in shared memory; per column the CTAs publish their
+//   * four 32-column panels, each factored by one kernel: up to 8192 rows one thread-block
+//     cluster with the rows in registers (below); above, a cooperative kernel whose CTAs
+//     keep slices of the panel's rows in shared memory; per column the CTAs publish their
 //     partial products of the column with all panel columns (which give the norm below
 //     the diagonal and, after the scaling, both the reflector's effect on the columns to
 //     its right and the dlarft vector for the columns to its left), one grid barrier, and
@@ -19,7 +20,7 @@
 //     writes the reflectors as an explicit unit lower trapezoid Y (zeros above) and the T
 //     block with zeros below its diagonal, so that every later product is a plain GEMM;
 //   * after each panel: the rest of the 128-column block takes the panel's reflectors
-//     (W = C^T Y_p by a split-K kernel pair, W = W T_p, C -= Y_p W^T);
+//     (W = C^T Y_p, its K split over the device, W = W T_p, C -= Y_p W^T);
 //   * after each block: its T (the four panel T blocks joined through Y_b^T Y_b by one CTA),
 //     T's rows above it, -T(0:kb,0:kb) (Y(:,0:kb)^T Y_b) T_b, and the columns to its right
 //     take Q_b^T in three products with K = 128 (W = C^T Y_b, W = W T_b, C -= Y_b W^T).
@@ -36,7 +37,9 @@
 // algorithm as the reference wherever that GEMV takes one block).
 #include <algorithm>
 
+#include "cluster.cuh"
 #include "context.cuh"
+#include "tri.cuh"
 
 namespace mo {
 namespace {
@@ -235,110 +238,248 @@ __global__ void __launch_bounds__(kQrThreads, 1)
     }
 }
 
+// ---- the panel in one thread-block cluster ---------------------------------------------
+// The panel is a chain of columns; with a grid barrier and two L2 round trips a column costs 4.6
+// us (8000 rows).  Here up to 16 CTAs x 256 threads x 2 rows hold the panel in registers and
+// exchange a column's products through distributed shared memory: every CTA sends its 32 sums,
+// and CTA 0 the pivot row, onto the others' mbarriers, and every CTA adds the sums in the same
+// order.  The loop over the columns is rolled and the registers rotate by one column per turn
+// (x[q][0] is the current one, finished columns come to the end), so that its instructions
+// stay in the cache; finished columns take part in the products (the dlarft vector) with a
+// zero update.  T follows from the kept vectors when the columns are done.
+// Measured on B200, 32 columns of 8000 to 6000 rows: 148 -> 93 us (of a column's 4.7 K cycles the
+// products and their warp sums take 1.3 K, the exchange 1.7 K, the scalars 0.5 K, the update 0.6 K).
+constexpr int kClThreads = 256, kClWarps = kClThreads / 32, kClMaxCtas = 16;
+constexpr int kClMaxRows = kClThreads * kClMaxCtas * 2;
+
+struct ClQr {
+  uint64_t bar[2];                 // arrival of a column's sums, by column parity
+  __align__(16) double sum[2][kClMaxCtas][32];
+  __align__(16) double prow[2][32];
+  __align__(16) double own[32], ownrow[32];  // gathered for sending
+  double red[kClWarps][32];
+  __align__(16) double w[kClWarps][32];      // each warp's copy of the update row
+  double z[32][33];                // dlarft vectors: z[j][c] = -tau_j v_c^T v_j, c < j
+  double tau[32];
+  double t[32][33];                // T, column j at t[j]
+};
+
+template <int RPT>
+__global__ void __launch_bounds__(kClThreads, 1)
+    qr_cluster_panel_kernel(double *P, int64_t ldp, int R, int w, double *Y, int64_t ldy, double *Tb,
+                            int64_t ldt, int *status) {
+  __shared__ ClQr s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nctas = gridDim.x, cta = blockIdx.x;  // one cluster: the grid is the cluster
+  const int rbase = cta * kClThreads * RPT + tid;  // rows rbase + kClThreads q
+  const int kmax = min(R, w);
+  double x[RPT][32];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = rbase + kClThreads * q;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) x[q][k] = r < R && k < w ? P[r + (int64_t)k * ldp] : 0.0;
+  }
+  if (tid == 0) {
+    mbar_init(&s.bar[0], 1);
+    mbar_init(&s.bar[1], 1);
+    fence_barrier_init();
+  }
+  if (nctas > 1) cl_sync();  // every CTA has started before any writes into its memory
+  else __syncthreads();
+#pragma unroll 1
+  for (int j = 0; j < kmax; ++j) {
+    const int par = j & 1;
+    // products of the current column with all 32 over the rows below j
+    double acc[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) acc[k] = 0.0;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int r = rbase + kClThreads * q;
+      if (r > j) {  // (rows past R hold zeros)
+#pragma unroll
+        for (int k = 0; k < 32; ++k) acc[k] = fma(x[q][0], x[q][k], acc[k]);
+      }
+    }
+    // the warp's 32 sums over its 32 lanes: lane l ends with column l's
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < o; ++k) {
+        const bool up = lane & o;
+        const double give = up ? acc[k] : acc[k + o], keep = up ? acc[k + o] : acc[k];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    s.red[warp][lane] = acc[0];
+    if (nctas > 1 && tid == 0)
+      mbar_arrive_expect_tx(&s.bar[par], (uint32_t)((nctas + 1) * 32 * sizeof(double)));
+    // the pivot row (one of CTA 0's first 32) goes out beside the sums
+    if (cta == 0 && warp == 0) {
+      double *to = nctas > 1 ? s.ownrow : s.prow[par];
+      if (tid == j) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) to[k] = x[0][k];
+      }
+      __syncwarp();
+      if (nctas > 1) cl_send<16>(s.prow[par], s.ownrow, &s.bar[par], lane, nctas);
+    }
+    __syncthreads();
+    double qv = 0.0;  // column `lane` (rotated index) over all rows below j
+    if (nctas > 1) {
+      if (warp == 1) {
+#pragma unroll
+        for (int g = 0; g < kClWarps; ++g) qv += s.red[g][lane];
+        s.own[lane] = qv;
+        __syncwarp();
+        cl_send<16>(s.sum[par][cta], s.own, &s.bar[par], lane, nctas);
+      }
+      // (a wait that runs out is recorded; the kernel goes on with what it holds)
+      mbar_wait(&s.bar[par], (j >> 1) & 1, status);
+      double part[kClMaxCtas];  // all loads in flight, added in order
+#pragma unroll
+      for (int g = 0; g < kClMaxCtas; ++g) part[g] = g < nctas ? s.sum[par][g][lane] : 0.0;
+      qv = 0.0;
+#pragma unroll
+      for (int g = 0; g < kClMaxCtas; ++g) qv += part[g];
+    } else {
+#pragma unroll
+      for (int g = 0; g < kClWarps; ++g) qv += s.red[g][lane];
+    }
+    const double prc = s.prow[par][lane];
+    // computeHouseholder (house.go:55-78) on [alpha; x] with ||x||^2 = q_0, in every lane
+    const double nrm2 = __shfl_sync(0xffffffffu, qv, 0), alpha = __shfl_sync(0xffffffffu, prc, 0);
+    double tau = 0.0, denom = 1.0, beta = alpha;
+    if (nrm2 != 0.0) {
+      // (the plain root of the sum where neither square leaves the normal range: the scaled
+      // one is two roots and a quotient, 500 cycles, on the chain)
+      const double a2 = alpha * alpha, ss = a2 + nrm2;
+      const double nrm = ss < 1e300 && nrm2 > 1e-280 ? sqrt(fma(alpha, alpha, nrm2))
+                                                     : qr_hypot(alpha, sqrt(nrm2));
+      beta = signbit(alpha) ? nrm : -nrm;
+      denom = alpha - beta;
+      tau = (beta - alpha) / beta;
+    }
+    // p_c = row j + v^T (rows below j) of column c, with v = x / denom; rotated index k is
+    // column j + k, finished ones (columns < j) at k >= 32 - j
+    const double p = tau != 0.0 ? tau * (prc + qv / denom) : 0.0;
+    s.w[warp][lane] = lane < 32 - j ? p : 0.0;
+    if (cta == 0 && warp == 2) {
+      if (lane >= 32 - j) s.z[j][lane - (32 - j)] = -p;
+      if (lane == 0) s.tau[j] = tau;
+    }
+    // with an infinity or a NaN about, finished rows and columns must not meet it even times zero
+    const bool odd = __any_sync(0xffffffffu, !isfinite(p) || !isfinite(qv));
+    __syncwarp();
+    // H(j) on this thread's rows: v = x / denom, rows below j lose v w, row j loses w and
+    // takes beta; the registers rotate
+    double v[RPT], last[RPT];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int r = rbase + kClThreads * q;
+      const double xv = tau != 0.0 ? x[q][0] / denom : x[q][0];
+      v[q] = r > j ? xv : (r == j ? 1.0 : 0.0);
+      last[q] = r > j ? xv : (r == j ? beta : x[q][0]);
+    }
+    if (odd) {
+#pragma unroll
+      for (int k = 1; k < 32; ++k)
+#pragma unroll
+        for (int q = 0; q < RPT; ++q)
+          x[q][k - 1] = k < 32 - j && rbase + kClThreads * q >= j ? fma(-v[q], s.w[warp][k], x[q][k])
+                                                                : x[q][k];
+    } else
+#pragma unroll
+    for (int k = 0; k < 32; k += 2) {
+      const double2 wk = *reinterpret_cast<const double2 *>(&s.w[warp][k]);
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        if (k > 0) x[q][k - 1] = fma(-v[q], wk.x, x[q][k]);
+        x[q][k] = fma(-v[q], wk.y, x[q][k + 1]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) x[q][31] = last[q];
+  }
+  // write back: R and the reflectors into P, the explicit Y (register k: column (k + kmax) % 32)
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = rbase + kClThreads * q;
+    if (r >= R) continue;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const int c = (k + kmax) & 31;
+      if (c >= w) continue;
+      P[r + (int64_t)c * ldp] = x[q][k];
+      Y[r + (int64_t)c * ldy] = r > c ? x[q][k] : (r == c ? 1.0 : 0.0);
+    }
+  }
+  __syncthreads();
+  if (cta == 0 && warp == 0) {
+    // T(0:j, j) = T(0:j, 0:j) z_j, T(j, j) = tau_j (zero column when tau == 0)
+    for (int j = 0; j < 32; ++j) {
+      double t = 0.0;
+      const double tau = j < kmax ? s.tau[j] : 0.0;
+      if (tau != 0.0 && lane < j)
+        for (int c = lane; c < j; ++c) t = fma(s.t[c][lane], s.z[j][c], t);
+      s.t[j][lane] = lane < j ? t : (lane == j ? tau : 0.0);
+      __syncwarp();
+    }
+    for (int c = 0; c < w; ++c)
+      if (lane < w) Tb[lane + (int64_t)c * ldt] = s.t[c][lane];
+  }
+  if (nctas > 1) cl_sync();  // no CTA leaves while another may still write into its memory
+}
+
 // The 128-column block's T from its four 32 x 32 panel blocks (on the diagonal of Tb, ld
 // ldt, zeros below) and the Gram matrix Zin = Y_b^T Y_b (ld ldz): for panel p the rows above
 // it are T(0:32p, p) = -T(0:32p, 0:32p) Zin(0:32p, p) T_pp (qrwy.go:433-453 at panel
 // granularity).  One CTA; the block lives in shared memory.
-constexpr int kQrTBlockSmem = (128 * 129 + 96 * 33) * 8;
+// Both products run as 16 x 16 tiles on the FP64 tensor pipe, a warp per tile: 78 us a block with
+// one FMA chain per element, 41 us this way.
+constexpr int kTbLd = 132;  // T(r, c) at r * kTbLd + c (4 mod 16: fragments without conflicts)
+constexpr int kQrTBlockSmem = (128 * kTbLd + 96 * 36) * 8;
 __global__ void __launch_bounds__(256) qr_t_block_kernel(double *Tb, int64_t ldt,
                                                          const double *Zin, int64_t ldz, int bo) {
   extern __shared__ double sm[];
-  double *T = sm;               // [128][129], T(r, c) at c * 129 + r
-  double *M1 = sm + 128 * 129;  // [32][33] x rows: M1(r, c) at c * 97 + r (r < 96)
-  const int tid = threadIdx.x;
-  for (int e = tid; e < bo * bo; e += 256) {
-    const int c = e / bo, r = e - c * bo;
-    T[c * 129 + r] = Tb[r + (int64_t)c * ldt];
+  double *T = sm;                  // [128][kTbLd], zeros outside bo x bo and below the diagonal
+  double *M1 = sm + 128 * kTbLd;   // [96][36]
+  const int tid = threadIdx.x, warp = tid >> 5;
+#pragma unroll 16
+  for (int e = tid; e < 128 * 128; e += 256) {
+    const int r = e & 127, c = e >> 7;
+    const bool own = r < bo && c < bo && r <= c && r / kQrPanel == c / kQrPanel;
+    // above the diagonal panels: the Gram matrix, replaced block column by block column
+    const bool gram = r < bo && c < bo && r / kQrPanel < c / kQrPanel;
+    T[r * kTbLd + c] = own ? Tb[r + (int64_t)c * ldt] : gram ? Zin[r + (int64_t)c * ldz] : 0.0;
   }
   __syncthreads();
   for (int p0 = kQrPanel; p0 < bo; p0 += kQrPanel) {
-    const int w = min(kQrPanel, bo - p0), R = p0;
-    // M1 = Zin(0:R, p0:p0+w) T(p0:p0+w, p0:p0+w)
-    for (int e = tid; e < R * w; e += 256) {
-      const int c = e / R, r = e - c * R;
-      double acc = 0.0;
-      for (int l = 0; l <= c; ++l)
-        acc = fma(Zin[r + (int64_t)(p0 + l) * ldz], T[(p0 + c) * 129 + p0 + l], acc);
-      M1[c * 97 + r] = acc;
+    const int nt = p0 / 16;  // 16-row tiles above the panel, two columns of them
+    // M1 = Zin(0:p0, p0:p0+32) T(p0:p0+32, p0:p0+32)
+    for (int t = warp; t < 2 * nt; t += 8) {
+      const int i = 16 * (t >> 1), j = 16 * (t & 1);
+      double c[2][4] = {};
+      for (int k = 0; k < kQrPanel; k += 16)
+        tri_mm16(c, T + i * kTbLd + p0 + k, kTbLd, 1, T + (p0 + k) * kTbLd + p0 + j, 1, kTbLd);
+      tri_put16(c, M1 + i * 36 + j, 36, 1, 1.0, false);
     }
     __syncthreads();
-    // T(0:R, p0:p0+w) = -T(0:R, 0:R) M1  (T upper triangular)
-    for (int e = tid; e < R * w; e += 256) {
-      const int c = e / R, r = e - c * R;
-      double acc = 0.0;
-      for (int l = r; l < R; ++l) acc = fma(T[l * 129 + r], M1[c * 97 + l], acc);
-      T[(p0 + c) * 129 + r] = -acc;
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < bo * bo; e += 256) {
-    const int c = e / bo, r = e - c * bo;
-    if (r < (c / kQrPanel) * kQrPanel) Tb[r + (int64_t)c * ldt] = T[c * 129 + r];
-  }
-}
-
-// Split-K product for a small C with a long K: C (M x N) = A^T B, A (K x M) and B (K x N)
-// column-major.  Grid (chunks, tiles): each CTA multiplies one chunk of K rows for one
-// 64 x 64 tile of C (16 x 16 threads, 4 x 4 outputs each, 32-row slabs staged in shared
-// memory) and stores its partial tile; tn_reduce_kernel sums the chunks in order.  The
-// engine would run such a product as one 128 x 128 tile whose K is split over ~100 CTAs
-// and summed by one of them.
-constexpr int kTnTile = 64, kTnSlab = 32;
-__global__ void __launch_bounds__(256) tn_partial_kernel(const double *A, int64_t lda,
-                                                         const double *B, int64_t ldb, int M,
-                                                         int N, int K, int kc, double *part) {
-  __shared__ double As[kTnSlab][kTnTile + 1], Bs[kTnSlab][kTnTile + 1];
-  const int tiles_m = (M + kTnTile - 1) / kTnTile;
-  const int tile = blockIdx.y, tm = tile % tiles_m, tn = tile / tiles_m;
-  const int m0 = tm * kTnTile, n0 = tn * kTnTile;
-  const int k_begin = blockIdx.x * kc, k_end = min(K, k_begin + kc);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  double acc[4][4] = {};
-  for (int k0 = k_begin; k0 < k_end; k0 += kTnSlab) {
-    // slab rows k0..k0+31 of A's columns m0.. and B's columns n0.. (zeros past the edges)
-    for (int e = tid; e < kTnSlab * kTnTile; e += 256) {
-      const int kk = e & (kTnSlab - 1), c = e / kTnSlab;
-      const int k = k0 + kk;
-      As[kk][c] = (k < k_end && m0 + c < M) ? A[k + (int64_t)(m0 + c) * lda] : 0.0;
-      Bs[kk][c] = (k < k_end && n0 + c < N) ? B[k + (int64_t)(n0 + c) * ldb] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < kTnSlab; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+    // T(0:p0, p0:p0+32) = -T(0:p0, 0:p0) M1  (T upper triangular)
+    for (int t = warp; t < 2 * nt; t += 8) {
+      const int i = 16 * (t >> 1), j = 16 * (t & 1);
+      double c[2][4] = {};
+      for (int k = i; k < p0; k += 16)
+        tri_mm16(c, T + i * kTbLd + k, kTbLd, 1, M1 + k * 36 + j, 1, 36);
+      tri_put16(c, T + i * kTbLd + p0 + j, kTbLd, 1, -1.0, false);
     }
     __syncthreads();
   }
-  double *out = part + ((size_t)blockIdx.x * gridDim.y + tile) * (kTnTile * kTnTile);
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[(ty + 16 * i) + (tx + 16 * j) * kTnTile] = acc[i][j];
-}
-
-// C = alpha * (sum of the chunks' partial tiles, in chunk order) + beta * C (beta == 0: C
-// not read)
-__global__ void __launch_bounds__(256) tn_reduce_kernel(const double *part, int chunks, int tiles,
-                                                        int M, int N, double *C, int64_t ldc,
-                                                        double alpha, double beta) {
-  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (e >= (int64_t)M * N) return;
-  const int i = (int)(e % M), j = (int)(e / M);
-  const int tiles_m = (M + kTnTile - 1) / kTnTile;
-  const int tile = (i / kTnTile) + (j / kTnTile) * tiles_m;
-  const int off = (i % kTnTile) + (j % kTnTile) * kTnTile;
-  double s = 0.0;
-  for (int c = 0; c < chunks; ++c) s += part[((size_t)c * tiles + tile) * (kTnTile * kTnTile) + off];
-  double *cp = C + i + (int64_t)j * ldc;
-  *cp = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *cp);
+  for (int e = tid; e < 128 * 128; e += 256) {
+    const int r = e & 127, c = e >> 7;
+    if (c < bo && r < (c / kQrPanel) * kQrPanel) Tb[r + (int64_t)c * ldt] = T[r * kTbLd + c];
+  }
 }
 
 // Y (m x k) = the explicit unit lower trapezoid of A's reflectors (zeros above)
@@ -419,6 +560,7 @@ struct QrWork {
   double *Z = nullptr;   // k x 128
   double *X = nullptr;   // k x 128
   QrScratch sc{};
+  int cl_rows = 0;       // rows up to which a panel runs in one cluster
 };
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -472,9 +614,61 @@ int max_panel_rows(mo_ctx *ctx) {
   return rpc * ctx->sms;
 }
 
+const void *cl_kernel(int rpt) {
+  return rpt == 1 ? (const void *)qr_cluster_panel_kernel<1> : (const void *)qr_cluster_panel_kernel<2>;
+}
+
+int cl_config(int ctas, int rpt, cudaStream_t st, cudaLaunchConfig_t *cfg,
+              cudaLaunchAttribute *attr) {
+  MO_CUDA_TRY(cudaFuncSetAttribute(cl_kernel(rpt), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(ctas);
+  cfg->blockDim = dim3(kClThreads);
+  cfg->stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim = {(unsigned)ctas, 1, 1};
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  return MO_OK;
+}
+
+// rows up to which a panel may run in one cluster (16 CTAs are not portable: ask)
+int cluster_rows(mo_ctx *ctx, int m, int *rows) {
+  *rows = kClThreads * 8;
+  if (m <= *rows) return MO_OK;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  int clusters = 0;
+  if (int rc = cl_config(kClMaxCtas, 2, ctx->stream, &cfg, &attr)) return rc;
+  if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(2), &cfg) == cudaSuccess && clusters > 0)
+    *rows = kClMaxRows;
+  else
+    cudaGetLastError();
+  return MO_OK;
+}
+
 // factor A[kp:m, kp:kp+bp]; its reflectors go to Y's and its T block to Tw's columns kp..
 int panel(mo_ctx *ctx, View A, int kp, int bp, QrWork &q, int k) {
   const int m = A.rows, R = m - kp;
+  if (R <= q.cl_rows) {
+    // one row per thread while 16 CTAs suffice
+    const int rpt = R > kClThreads * kClMaxCtas ? 2 : 1;
+    int ctas = 1;
+    while (ctas * kClThreads * rpt < R) ctas *= 2;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    if (int rc = cl_config(ctas, rpt, ctx->stream, &cfg, &attr)) return rc;
+    double *P = A.at(kp, kp), *Y = q.Y + kp + (int64_t)kp * m, *Tb = q.Tw + kp + (int64_t)kp * k;
+    int64_t ldp = A.ld, ldy = m, ldt = k;
+    int rows = R, w = bp, *status = &control(ctx)->status;
+    void *args[] = {&P, &ldp, &rows, &w, &Y, &ldy, &Tb, &ldt, &status};
+    ProfScope ps;
+    prof_begin(ctx, ps, MO_PROF_PANEL);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, cl_kernel(rpt), args);
+    prof_end(ctx, ps, 4.0 * R * (double)bp * bp, 8.0 * 3 * R * (double)bp);
+    MO_CUDA_TRY(e);
+    return MO_OK;
+  }
   int grid = 0, rpc = 0;
   panel_shape(ctx, R, grid, rpc);
   const size_t smem = qr_panel_smem(rpc);
@@ -512,39 +706,13 @@ int t_columns(mo_ctx *ctx, int k, int kp, int bp, View Zsrc, QrWork &q) {
   return rc;
 }
 
-// C = alpha * A^T B + beta * C: split-K kernels when C is small and K long, else the
-// engine (its stream-K scratch doubles as the partial-tile buffer: same stream, in order)
-int tn_product(mo_ctx *ctx, View C, View A, View B, double alpha, double beta) {
-  const int M = C.rows, N = C.cols, K = A.rows;
-  if (M <= 0 || N <= 0) return MO_OK;
-  const int tiles = ((M + kTnTile - 1) / kTnTile) * ((N + kTnTile - 1) / kTnTile);
-  const size_t cap = gemm_partial_bytes(ctx->sms) / sizeof(double) / (kTnTile * kTnTile);
-  if (K < 1024 || tiles > 16 || K <= 0) return gemm(ctx, C, A, true, B, false, alpha, beta);
-  double *part = ctx->sk_partial;
-  // chunks of at least 128 rows, about two CTAs per SM, within the partial buffer
-  int chunks = std::max(1, std::min<int>(K / 128, (2 * ctx->sms + tiles - 1) / tiles));
-  chunks = std::min<int>(chunks, (int)(cap / tiles));
-  const int kc = ((K + chunks - 1) / chunks + kTnSlab - 1) / kTnSlab * kTnSlab;
-  chunks = (K + kc - 1) / kc;
-  ProfScope ps;
-  prof_begin(ctx, ps, MO_PROF_GEMM);
-  tn_partial_kernel<<<dim3(chunks, tiles), 256, 0, ctx->stream>>>(A.d, A.ld, B.d, B.ld, M, N, K,
-                                                                    kc, part);
-  const int64_t mn = (int64_t)M * N;
-  tn_reduce_kernel<<<(unsigned)((mn + 255) / 256), 256, 0, ctx->stream>>>(
-      part, chunks, tiles, M, N, C.d, C.ld, alpha, beta);
-  prof_end(ctx, ps, 2.0 * M * N * (double)K, 8.0 * ((double)K * (M + N) + 2.0 * M * N));
-  MO_CUDA_TRY(cudaGetLastError());
-  return MO_OK;
-}
-
 // C (rows s.. of A's columns right of a block) = Q_b^T C for the block's reflectors:
 // W = C^T Y_b, W = W T_b, C -= Y_b W^T (qrwy.go:266-303 with transpose)
 int apply_left_t(mo_ctx *ctx, View C, const View &Yb, const View &Tb, QrWork &q) {
   const int nc = C.cols, b = Yb.cols;
   if (nc <= 0 || b <= 0) return MO_OK;
   const View W{q.W, nc, b, nc}, W2{q.W2, nc, b, nc};
-  int rc = tn_product(ctx, W, C, Yb, 1.0, 0.0);
+  int rc = gemm(ctx, W, C, true, Yb, false, 1.0, 0.0);
   if (!rc) rc = gemm(ctx, W2, W, false, Tb, false, 1.0, 0.0);
   if (!rc) rc = gemm(ctx, C, Yb, false, W2, true, -1.0, 1.0);
   return rc;
@@ -591,7 +759,7 @@ int factor_block(mo_ctx *ctx, View A, int kb, int bo, int k, QrWork &q) {
   const View Yb = Yv.sub(kb, kb, m - kb, bo), Tb = Tv.sub(kb, kb, bo, bo);
   if (bo > kQrPanel) {
     const View Zin{q.W2, bo, bo, bo};
-    if ((rc = tn_product(ctx, Zin, Yb, Yb, 1.0, 0.0))) return rc;
+    if ((rc = gemm(ctx, Zin, Yb, true, Yb, false, 1.0, 0.0))) return rc;
     if ((rc = mo_smem_attr((const void *)qr_t_block_kernel, kQrTBlockSmem))) return rc;
     qr_t_block_kernel<<<1, 256, kQrTBlockSmem, ctx->stream>>>(Tb.d, k, q.W2, bo, bo);
     MO_CUDA_TRY(cudaGetLastError());
@@ -599,7 +767,7 @@ int factor_block(mo_ctx *ctx, View A, int kb, int bo, int k, QrWork &q) {
   if (kb > 0) {
     // T's rows above the block: -T(0:kb, 0:kb) (Y(kb:m, 0:kb)^T Y_b) T_b
     const View Z{q.Z, kb, bo, kb};
-    if ((rc = tn_product(ctx, Z, Yv.sub(kb, 0, m - kb, kb), Yb, 1.0, 0.0))) return rc;
+    if ((rc = gemm(ctx, Z, Yv.sub(kb, 0, m - kb, kb), true, Yb, false, 1.0, 0.0))) return rc;
     if ((rc = t_columns(ctx, k, kb, bo, Z, q))) return rc;
   }
   return MO_OK;
@@ -618,6 +786,7 @@ int qr_factor(mo_ctx *ctx, View A, View T, double *tau, int64_t tau_inc) {
   QrWork q;
   int rc = qr_workspace(ctx, m, k, (int64_t)max(n, 1) * kQrBlock, grid, q);
   if (rc) return rc;
+  if ((rc = cluster_rows(ctx, m, &q.cl_rows))) return rc;
   const View Yv{q.Y, m, k, m}, Tv{q.Tw, k, k, k};
   // the products read T's blocks below the diagonal and Y's rows above each panel inside
   // a 128-column block as zeros (the panels write only their own rows and T blocks)
@@ -673,7 +842,7 @@ int qr_apply(mo_ctx *ctx, View C, int m, int k, int flags, int nb, QrWork &q) {
     if (!right) {
       const int nc = C.cols;
       const View Cs = C.sub(s, 0, m - s, nc), W{q.W, nc, b, nc}, W2{q.W2, nc, b, nc};
-      int r = tn_product(ctx, W, Cs, Yb, 1.0, 0.0);
+      int r = gemm(ctx, W, Cs, true, Yb, false, 1.0, 0.0);
       if (!r) r = gemm(ctx, W2, W, false, Tb, !trans, 1.0, 0.0);
       if (!r) r = gemm(ctx, Cs, Yb, false, W2, true, -1.0, 1.0);
       return r;
