@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "context.cuh"
+#include "tri.cuh"
 
 namespace mo {
 int trtri_blocks(mo_ctx *ctx, View A, int N, bool trans, bool lower_eff, bool unit, double *inv);
@@ -170,16 +171,19 @@ int chol_adjoint_one(mo_ctx *ctx, View L, View G, const AdjScratch &w, bool stre
 }
 
 // ---------------------------------------------------------------------------------------
-// Batched form for orders up to kAdjBatchMaxN: one persistent kernel, each CTA takes whole
-// matrices from a longest-first queue and runs the same reverse sweep with 32-column
-// blocks inside the CTA: every product is a small GEMM over shared-memory tiles (FP64 FMA,
-// 4 outputs per thread), the 32 x 32 diagonal work (D^-1 and the adjoint of chol(D)) stays
-// in shared memory, and L and Lbar are read and written in place (they stay in L2 at these
-// orders).  One launch replaces the per-matrix chain of about 25 launches per block.
+// Batched form for orders up to kAdjBatchMaxN: one persistent kernel, each CTA of four warps takes
+// whole matrices from a longest-first queue and runs the same reverse sweep with 32-column
+// blocks.  The large products are 32 x 32 tiles on the FP64 tensor pipe, a warp each, their
+// fragments loaded straight from L and Lbar (which stay in L2 and L1 at these orders).  Warps 1
+// to 3 do Cbar -= Bbar R and Rbar -= Bbar^T C while warp 0 does what hangs together in a chain:
+// Dbar -= Bbar^T B, the adjoint of chol(D), and D^-1 of the next block.
+// What bounds it is that chain and the latency of the fragment loads; four CTAs per SM cover
+// each other.  Measured on B200, 512 x n = 256, factorization and reverse sweep: 2.37 -> 1.60 ms
+// (against FMA on tiles staged in shared memory, all warps in step; the sweep alone was 1.88).
 // ---------------------------------------------------------------------------------------
 constexpr int AB = 32;     // block columns per step
-constexpr int ABT = 256;   // threads per CTA
-constexpr int ALD = AB + 1;
+constexpr int ABT = 128;   // threads per CTA
+constexpr int ALD = AB + 4;  // 4 mod 16 doubles: fragments without bank conflicts
 constexpr int kAdjBatchMaxN = 512;
 
 struct AdjBatchArgs {
@@ -194,163 +198,206 @@ struct AdjBatchArgs {
 };
 
 struct AdjSmem {
-  double As[AB][ALD], Bs[AB][ALD];    // GEMM staging
-  double Dm[AB][ALD], Di[AB][ALD];    // D (lower, identity padded) and D^-1
-  double X1[AB][ALD], X2[AB][ALD];    // the adjoint of chol(D)
+  double D[AB * ALD], Di[AB * ALD];  // D (lower, identity padded) and D^-1, row-major
+  double X1[AB * ALD], X2[AB * ALD]; // the adjoint of chol(D); E = S + S^T ends in X1
   int idx;
 };
 
-// C (M x N, ldc) += alpha op(A) op(B), op(A) M x K, op(B) K x N; `lower`: only i >= j.
-// op(A)(i, k) = ta ? A[k + i lda] : A[i + k lda]; op(B)(k, j) = tb ? B[j + k ldb] : B[k + j ldb].
-// C must not overlap A or B.  Ends with a barrier.
-__device__ void adj_gemm(AdjSmem &s, int M, int N, int K, double alpha, const double *A, int64_t lda,
-                         bool ta, const double *B, int64_t ldb, bool tb, double *C, int64_t ldc,
-                         bool lower) {
-  const int tid = threadIdx.x, r = tid & 31, cg = tid >> 5;  // row r, columns 4 cg .. + 3
-  for (int i0 = 0; i0 < M; i0 += AB)
-    for (int j0 = 0; j0 < N; j0 += AB) {
-      if (lower && j0 > i0 + AB - 1) continue;
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int k0 = 0; k0 < K; k0 += AB) {
-        __syncthreads();
-        for (int e = tid; e < AB * AB; e += ABT) {
-          const int a = e & 31, b = e >> 5;
-          const int ii = ta ? b : a, ka = ta ? a : b;  // consecutive threads: consecutive addresses
-          const int gi = i0 + ii, gk = k0 + ka;
-          s.As[ii][ka] = (gi < M && gk < K) ? (ta ? A[gk + (int64_t)gi * lda] : A[gi + (int64_t)gk * lda]) : 0.0;
-          const int kb = tb ? b : a, jj = tb ? a : b;
-          const int gk2 = k0 + kb, gj = j0 + jj;
-          s.Bs[kb][jj] = (gk2 < K && gj < N) ? (tb ? B[gj + (int64_t)gk2 * ldb] : B[gk2 + (int64_t)gj * ldb]) : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int k = 0; k < AB; ++k) {
-          const double av = s.As[r][k];
+// acc (32 x 32: rows 16 mi + g + 8 h, columns 8 ni + 2 t + e at acc[mi][ni][2 h + e]) +=
+// sum over k < K of P(i, k) Q(k, j) with P(i, k) = p[i * pi + k * pk], Q(k, j) = q[k * qk + j * qj];
+// rows past M and columns past N are computed from the last one
+__device__ __forceinline__ void adj_tile(double (&acc)[2][4][4], int M, int N, int K, const double *p,
+                                         int64_t pi, int64_t pk, const double *q, int64_t qk,
+                                         int64_t qj) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const double *pa[2][2], *pb[4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[c] = fma(av, s.Bs[k][4 * cg + c], acc[c]);
-        }
-      }
+  for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int gi = i0 + r, gj = j0 + 4 * cg + c;
-        if (gi < M && gj < N && (!lower || gi >= gj)) C[gi + (int64_t)gj * ldc] += alpha * acc[c];
-      }
-    }
-  __syncthreads();
+    for (int h = 0; h < 2; ++h) pa[mi][h] = p + min(16 * mi + 8 * h + g, M - 1) * pi + t * pk;
+#pragma unroll
+  for (int ni = 0; ni < 4; ++ni) pb[ni] = q + min(8 * ni + g, N - 1) * qj + t * qk;
+  double a[2][2], b[4];
+  auto load = [&](int k, double (&x)[2][2], double (&y)[4]) {
+    const bool in = k + t < K;
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) x[mi][h] = in ? pa[mi][h][k * pk] : 0.0;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) y[ni] = in ? pb[ni][k * qk] : 0.0;
+  };
+  if (K <= 0) return;
+  load(0, a, b);
+#pragma unroll 1
+  for (int k = 0; k < K; k += 4) {
+    double an[2][2], bn[4];
+    load(k + 4, an, bn);
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) dmma_16x8x4(acc[mi][ni], a[mi][0], a[mi][1], b[ni]);
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) a[mi][h] = an[mi][h];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) b[ni] = bn[ni];
+  }
 }
 
-// Z = op(X) op(Y) for 32 x 32 shared-memory blocks (Z distinct from X and Y); ends with a barrier
-__device__ void adj_mm32(double (*Z)[ALD], const double (*X)[ALD], bool tx, const double (*Y)[ALD],
-                         bool ty) {
-  const int tid = threadIdx.x, r = tid & 31, cg = tid >> 5;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+// f(row, column, value) for every element of the tile that lies in M x N
+template <typename F>
+__device__ __forceinline__ void adj_each(const double (&acc)[2][4][4], int M, int N, F &&f) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = 16 * mi + g + 8 * (q >> 1), j = 8 * ni + 2 * t + (q & 1);
+        if (i < M && j < N) f(i, j, acc[mi][ni][q]);
+      }
+}
+
+// Z = op(X) op(Y) for 32 x 32 shared-memory blocks (Z distinct from X and Y), one warp
+__device__ __forceinline__ void adj_mm32(double *Z, const double *X, bool tx, const double *Y, bool ty) {
+  double acc[2][4][4] = {};
+  adj_tile(acc, AB, AB, AB, X, tx ? 1 : ALD, tx ? ALD : 1, Y, ty ? 1 : ALD, ty ? ALD : 1);
+  adj_each(acc, AB, AB, [&](int i, int j, double v) { Z[i * ALD + j] = v; });
+  __syncwarp();
+}
+
+// D of the block at j0 and its inverse, by one warp (identity padding past jb)
+__device__ __noinline__ void adj_diag(AdjSmem &s, const double *L, int64_t ldl, int j0, int jb) {
+  const int lane = threadIdx.x & 31;
+  const double *D = L + j0 + (int64_t)j0 * ldl;
 #pragma unroll 8
-  for (int k = 0; k < AB; ++k) {
-    const double xv = tx ? X[k][r] : X[r][k];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c] = fma(xv, ty ? Y[4 * cg + c][k] : Y[k][4 * cg + c], acc[c]);
+  for (int j = 0; j < AB; ++j) {
+    s.D[lane * ALD + j] =
+        (lane < jb && j < jb) ? (lane >= j ? D[lane + (int64_t)j * ldl] : 0.0) : (lane == j ? 1.0 : 0.0);
+    s.Di[lane * ALD + j] = 0.0;
   }
-#pragma unroll
-  for (int c = 0; c < 4; ++c) Z[r][4 * cg + c] = acc[c];
-  __syncthreads();
+  __syncwarp();
+  for (int h = 0; h < AB; h += 16) {
+    const double *B = s.D + h * (ALD + 1);
+    tri_inv16(s.Di + h * (ALD + 1), 1, ALD, 1.0 / B[(lane & 15) * (ALD + 1)],
+              [&](int i, int m) { return B[i * ALD + m]; });
+  }
+  __syncwarp();
+  // X21 = -X22 (L21 X11), the inner product through the (zero) upper right block of Di
+  double c[2][4] = {};
+  tri_mm16(c, s.D + 16 * ALD, ALD, 1, s.Di, 1, ALD);
+  tri_put16(c, s.Di + 16, ALD, 1, 1.0, false);
+  double x[2][4] = {};
+  tri_mm16(x, s.Di + 16 * (ALD + 1), ALD, 1, s.Di + 16, 1, ALD);
+  tri_put16(x, s.Di + 16 * ALD, ALD, 1, -1.0, false);
+  for (int i = 0; i < 16; ++i)
+    if (lane >= 16) s.Di[i * ALD + lane] = 0.0;
+  __syncwarp();
 }
 
 // the reverse sweep of one matrix (order n <= kAdjBatchMaxN) by the whole CTA
 __device__ void adj_matrix(AdjSmem &s, const double *L, int64_t ldl, double *G, int64_t ldg, int n) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int last = ((n - 1) / AB) * AB;
+  if (warp == 0) adj_diag(s, L, ldl, last, n - last);
   for (int j0 = last; j0 >= 0; j0 -= AB) {
-    const int jb = min(AB, n - j0), below = n - j0 - jb;
-    const double *D = L + j0 + (int64_t)j0 * ldl;
+    const int jb = min(AB, n - j0), below = n - j0 - jb, r1 = j0 + jb;
     double *Dbar = G + j0 + (int64_t)j0 * ldg;
-    for (int e = tid; e < AB * AB; e += ABT) {
-      const int i = e & 31, j = e >> 5;
-      s.Dm[i][j] = (i < jb && j < jb) ? (i >= j ? D[i + (int64_t)j * ldl] : 0.0) : (i == j ? 1.0 : 0.0);
+    double *Bbar = G + r1 + (int64_t)j0 * ldg;
+    const double *B = L + r1 + (int64_t)j0 * ldl;
+    __syncthreads();  // D^-1 is there, the previous step's updates are stored
+    // Bbar <- Bbar D^-1, 32 rows per warp (a tile is read before it is written)
+    for (int i0 = AB * warp; i0 < below; i0 += AB * (ABT / 32)) {
+      double acc[2][4][4] = {};
+      adj_tile(acc, below - i0, jb, jb, Bbar + i0, 1, ldg, s.Di, ALD, 1);
+      __syncwarp();
+      adj_each(acc, below - i0, jb,
+               [&](int i, int j, double v) { Bbar[i0 + i + (int64_t)j * ldg] = v; });
     }
     __syncthreads();
-    // D^-1 (lower): lane c of warp 0 solves D x = e_c
     if (warp == 0) {
-      const double rdi = 1.0 / s.Dm[lane][lane];
-      double x[AB];
-#pragma unroll
+      // X1 = tril(Dbar - Bbar^T B)
+      double acc[2][4][4] = {};
+      adj_tile(acc, jb, jb, below, Bbar, ldg, 1, B, 1, ldl);
+      adj_each(acc, AB, AB, [&](int i, int j, double v) {
+        s.X1[i * ALD + j] = (i < jb && j < jb && i >= j) ? Dbar[i + (int64_t)j * ldg] - v : 0.0;
+      });
+      __syncwarp();
+      // adjoint of chol(D): S = D^-T Phi(D^T X1) D^-1
+      adj_mm32(s.X2, s.D, true, s.X1, false);
       for (int i = 0; i < AB; ++i) {
-        double s0 = (i == lane) ? 1.0 : 0.0, s1 = 0.0;
-#pragma unroll
-        for (int m = 0; m + 1 < i; m += 2) {
-          s0 = fma(-s.Dm[i][m], x[m], s0);
-          s1 = fma(-s.Dm[i][m + 1], x[m + 1], s1);
-        }
-        if (i & 1) s0 = fma(-s.Dm[i][i - 1], x[i - 1], s0);
-        const double rd = __shfl_sync(0xffffffffu, rdi, i);
-        x[i] = (i < lane) ? 0.0 : (s0 + s1) * rd;
+        const double v = s.X2[i * ALD + lane];
+        s.X2[i * ALD + lane] = i > lane ? v : (i == lane ? 0.5 * v : 0.0);
       }
-#pragma unroll
-      for (int i = 0; i < AB; ++i) s.Di[i][lane] = x[i];
-    }
-    __syncthreads();
-    if (below > 0) {
-      double *Bbar = G + (j0 + jb) + (int64_t)j0 * ldg;
-      const double *B = L + (j0 + jb) + (int64_t)j0 * ldl;
-      // Bbar <- Bbar D^-1 in 32-row chunks through the staging tiles
-      for (int r0 = 0; r0 < below; r0 += AB) {
-        for (int e = tid; e < AB * AB; e += ABT) {
-          const int i = e & 31, k = e >> 5;
-          s.As[i][k] = (r0 + i < below && k < jb) ? Bbar[(r0 + i) + (int64_t)k * ldg] : 0.0;
-        }
-        __syncthreads();
-        adj_mm32(s.Bs, s.As, false, s.Di, false);
-        for (int e = tid; e < AB * AB; e += ABT) {
-          const int i = e & 31, j = e >> 5;
-          if (r0 + i < below && j < jb) Bbar[(r0 + i) + (int64_t)j * ldg] = s.Bs[i][j];
-        }
-        __syncthreads();
+      __syncwarp();
+      adj_mm32(s.X1, s.X2, false, s.Di, false);
+      adj_mm32(s.X2, s.Di, true, s.X1, false);
+      // E = S + S^T into X1; Dbar (lower) = Phi of it
+      for (int j = 0; j < AB; ++j) {
+        const double v = s.X2[lane * ALD + j] + s.X2[j * ALD + lane];
+        s.X1[lane * ALD + j] = v;
+        if (lane < jb && j < jb && lane >= j) Dbar[lane + (int64_t)j * ldg] = lane == j ? 0.5 * v : v;
       }
-      adj_gemm(s, jb, jb, below, -1.0, Bbar, ldg, true, B, ldl, false, Dbar, ldg, true);
-      if (j0 > 0) {
-        adj_gemm(s, below, j0, jb, -1.0, Bbar, ldg, false, L + j0, ldl, false, G + (j0 + jb), ldg,
-                 false);  // Cbar -= Bbar R
-        adj_gemm(s, jb, j0, below, -1.0, Bbar, ldg, true, L + (j0 + jb), ldl, false, G + j0, ldg,
-                 false);  // Rbar -= Bbar^T C
+      __syncwarp();
+      if (j0 > 0) adj_diag(s, L, ldl, j0 - AB, AB);
+    } else if (j0 > 0) {
+      const int nj = j0 / AB, ni = (below + AB - 1) / AB;
+      for (int t = warp - 1; t < nj * (ni + 1); t += ABT / 32 - 1) {
+        const int jt = t % nj * AB;
+        double acc[2][4][4] = {};
+        if (t < nj) {  // Rbar -= Bbar^T C, the long ones first
+          adj_tile(acc, jb, AB, below, Bbar, ldg, 1, L + r1 + (int64_t)jt * ldl, 1, ldl);
+          adj_each(acc, jb, AB,
+                   [&](int i, int j, double v) { G[j0 + i + (int64_t)(jt + j) * ldg] -= v; });
+        } else {       // Cbar -= Bbar R
+          const int it = (t / nj - 1) * AB;
+          adj_tile(acc, below - it, AB, jb, Bbar + it, 1, ldg, L + j0 + (int64_t)jt * ldl, 1, ldl);
+          adj_each(acc, below - it, AB,
+                   [&](int i, int j, double v) { G[r1 + it + i + (int64_t)(jt + j) * ldg] -= v; });
+        }
       }
     }
-    // adjoint of chol(D): S = D^-T Phi(D^T tril(Dbar)) D^-1
-    for (int e = tid; e < AB * AB; e += ABT) {
-      const int i = e & 31, j = e >> 5;
-      s.X1[i][j] = (i < jb && j < jb && i >= j) ? Dbar[i + (int64_t)j * ldg] : 0.0;
-    }
     __syncthreads();
-    adj_mm32(s.X2, s.Dm, true, s.X1, false);
-    for (int e = tid; e < AB * AB; e += ABT) {
-      const int i = e & 31, j = e >> 5;
-      s.X2[i][j] = i > j ? s.X2[i][j] : (i == j ? 0.5 * s.X2[i][j] : 0.0);
+    // Rbar -= E R
+    for (int jt = AB * warp; jt < j0; jt += AB * (ABT / 32)) {
+      double acc[2][4][4] = {};
+      adj_tile(acc, jb, AB, jb, s.X1, ALD, 1, L + j0 + (int64_t)jt * ldl, 1, ldl);
+      adj_each(acc, jb, AB,
+               [&](int i, int j, double v) { G[j0 + i + (int64_t)(jt + j) * ldg] -= v; });
     }
-    __syncthreads();
-    adj_mm32(s.X1, s.X2, false, s.Di, false);
-    adj_mm32(s.X2, s.Di, true, s.X1, false);
-    // E = S + S^T; Dbar (lower) = Phi-like copy of E
-    for (int e = tid; e < AB * AB; e += ABT) {
-      const int i = e & 31, j = e >> 5;
-      const double v = s.X2[i][j] + s.X2[j][i];
-      s.X1[i][j] = v;
-      if (i < jb && j < jb && i >= j) Dbar[i + (int64_t)j * ldg] = i == j ? 0.5 * v : v;
-    }
-    __syncthreads();
-    if (j0 > 0)  // Rbar -= E R
-      adj_gemm(s, jb, j0, jb, -1.0, &s.X1[0][0], ALD, true, L + j0, ldl, false, G + j0, ldg, false);
   }
-  // lower-entry adjoint -> symmetric gradient
-  for (int64_t e = tid; e < (int64_t)n * n; e += ABT) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    if (i > j) {
-      const double v = 0.5 * G[i + (int64_t)j * ldg];
-      G[i + (int64_t)j * ldg] = v;
-      G[j + (int64_t)i * ldg] = v;
+  __syncthreads();
+  // lower-entry adjoint -> symmetric gradient, a warp per 32 x 32 tile through its buffer
+  double *buf = s.D + warp * AB * ALD;
+  const int nt = (n + AB - 1) / AB;
+  for (int t = warp; t < nt * (nt + 1) / 2; t += ABT / 32) {
+    int bi = 0;
+    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+    const int i0 = AB * bi, j0 = AB * (t - bi * (bi + 1) / 2);
+    const int nr = min(AB, n - i0), nc = min(AB, n - j0);
+#pragma unroll 8
+    for (int j = 0; j < nc; ++j) {
+      const int i = i0 + lane, c = j0 + j;
+      double v = 0.0;
+      if (lane < nr && i >= c) {
+        v = G[i + (int64_t)c * ldg];
+        if (i > c) G[i + (int64_t)c * ldg] = v = 0.5 * v;
+      }
+      buf[j * ALD + lane] = v;
     }
+    __syncwarp();
+#pragma unroll 8
+    for (int i = 0; i < nr; ++i)
+      if (lane < nc && i0 + i > j0 + lane) G[(j0 + lane) + (int64_t)(i0 + i) * ldg] = buf[lane * ALD + i];
+    __syncwarp();
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(ABT) adj_batch_kernel(AdjBatchArgs p) {
+__global__ void __launch_bounds__(ABT, 4) adj_batch_kernel(AdjBatchArgs p) {
   extern __shared__ __align__(16) unsigned char adj_smem_raw[];
   AdjSmem &s = *reinterpret_cast<AdjSmem *>(adj_smem_raw);
   for (;;) {

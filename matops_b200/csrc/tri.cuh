@@ -127,9 +127,9 @@ __device__ __forceinline__ void tri_put16(const double (&c)[2][4], double *d, in
 }
 
 // Column c = lane % 16 of the inverse of a 16 x 16 lower triangle: L(i, m) for m < i through
-// l(i, m), reciprocal diagonal rd of row lane % 16; to Xd[c * XLD + i]
+// l(i, m), reciprocal diagonal rd of row lane % 16; X(i, c) to Xd[c * ldc + i * ldi]
 template <typename F>
-__device__ __forceinline__ void tri_inv16(double *Xd, double rd, F &&l) {
+__device__ __forceinline__ void tri_inv16(double *Xd, int ldc, int ldi, double rd, F &&l) {
   const int lane = threadIdx.x & 31, c = lane & 15;
   double x[16];
 #pragma unroll
@@ -145,7 +145,7 @@ __device__ __forceinline__ void tri_inv16(double *Xd, double rd, F &&l) {
   }
   if (lane < 16) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) Xd[c * XLD + i] = i < c ? 0.0 : x[i];
+    for (int i = 0; i < 16; ++i) Xd[c * ldc + i * ldi] = i < c ? 0.0 : x[i];
   }
 }
 
@@ -200,7 +200,7 @@ __device__ __forceinline__ int tri_potrf16(double *B, double *Xd, double *col, d
     for (int k = 0; k < 16; ++k)
       if (k <= i16) B[i16 * LDS + k] = k == i16 ? dg : r[k];
   }
-  tri_inv16(Xd, rd, [&](int i, int m) { return col[16 * m + i]; });
+  tri_inv16(Xd, XLD, 1, rd, [&](int i, int m) { return col[16 * m + i]; });
   __syncwarp();
   return -1;
 }
@@ -297,7 +297,7 @@ __device__ inline void tri_inverse_lower(const TriSmem &t, int NP) {
   if (warp < nb) {
     const double *B = t.S + 16 * warp * (LDS + 1);
     const double rd = 1.0 / B[(lane & 15) * (LDS + 1)];
-    tri_inv16(t.Xd + 16 * warp * XLD, rd, [&](int i, int m) { return B[i * LDS + m]; });
+    tri_inv16(t.Xd + 16 * warp * XLD, XLD, 1, rd, [&](int i, int m) { return B[i * LDS + m]; });
   }
   __syncthreads();
   for (int i = 1; i < nb; ++i) {
