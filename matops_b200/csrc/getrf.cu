@@ -763,25 +763,26 @@ __global__ void __launch_bounds__(256) swap_map_table_kernel(const int64_t *piv,
   if (threadIdx.x == 0) *count = total;
 }
 
-// A[dst[i], c] = A_old[src[i], c] for the moves of swap_map_kernel, columns [0, ncols): a
-// CTA takes 32 columns, loads every source row of them into shared memory (lanes along the
-// rows, so the contiguous block rows are read 256 bytes at a time), then stores.
-__global__ void __launch_bounds__(256) laswp_map_kernel(double *A, int64_t ld, int ncols,
-                                                        const int *dst, const int *src,
-                                                        const int *count) {
-  extern __shared__ double vals[];  // [count][32]
-  const int cnt = *count;
-  const int c0 = blockIdx.x * 32;
-  const int nc = min(32, ncols - c0);
-  for (int e = threadIdx.x; e < cnt * nc; e += blockDim.x) {
-    const int i = e % cnt, c = e / cnt;
-    vals[c * cnt + i] = A[src[i] + (int64_t)(c0 + c) * ld];
-  }
+// A[dst[i], c] = A_old[src[i], c] for a panel's moves, columns [0, ncols): a CTA takes 32 columns, a
+// thread one move (at most 2 MAX_PANEL_W of them), all its 32 loads in flight, then a barrier,
+// then the stores.  What bounds it at many columns is the scattered half of the rows, a 32-byte
+// sector per element (16384 columns: 130 us); 1001 columns take 7 us, 21 with a division per element and the values
+// passed through shared memory.
+__global__ void __launch_bounds__(2 * MAX_PANEL_W) laswp_map_kernel(double *A, int64_t ld, int ncols,
+                                                                    const int *dst, const int *src,
+                                                                    const int *count) {
+  const int i = threadIdx.x, c0 = blockIdx.x * 32;
+  const bool mine = i < *count;
+  double v[32];
+  const double *from = A + (mine ? src[i] : 0) + (int64_t)c0 * ld;
+#pragma unroll
+  for (int c = 0; c < 32; ++c) v[c] = mine && c0 + c < ncols ? from[c * ld] : 0.0;
   __syncthreads();
-  for (int e = threadIdx.x; e < cnt * nc; e += blockDim.x) {
-    const int i = e % cnt, c = e / cnt;
-    A[dst[i] + (int64_t)(c0 + c) * ld] = vals[c * cnt + i];
-  }
+  if (!mine) return;
+  double *to = A + dst[i] + (int64_t)c0 * ld;
+#pragma unroll
+  for (int c = 0; c < 32; ++c)
+    if (c0 + c < ncols) to[c * ld] = v[c];
 }
 
 // All interchanges rows s <-> piv[s] (s = 0 .. ns - 1, in order) on a few columns of B
@@ -792,22 +793,37 @@ __global__ void __launch_bounds__(256) laswp_cols_kernel(double *B, int64_t ld, 
   extern __shared__ double col[];
   double *g = B + (int64_t)blockIdx.x * ld;
   for (int i = threadIdx.x; i < rows; i += blockDim.x) col[i] = g[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < ns; ++s) {
-      const int64_t p = piv[s];
-      if (p <= 0 || p == s) continue;
-      if (p >= rows || s >= rows) {
-        if (blockIdx.x == 0) set_status(status, MO_EINVAL);
-        continue;
+  // the pivots come through shared memory, a part at a time (read one by one from global memory
+  // they set the pace: 240 cycles a swap); an entry that is not applied becomes its own row
+  constexpr int kPart = 1024;
+  __shared__ int part[kPart];
+  for (int s0 = 0; s0 < ns; s0 += kPart) {
+    const int np = min(kPart, ns - s0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+      const int64_t p = piv[s0 + i];
+      const bool out = p > 0 && p != s0 + i && (p >= rows || s0 + i >= rows);
+      if (out && blockIdx.x == 0) set_status(status, MO_EINVAL);
+      part[i] = p <= 0 || out ? s0 + i : (int)p;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < np; ++i) {
+        const int s = s0 + i, p = part[i];
+        if (p == s) continue;
+        const double t = col[s];
+        col[s] = col[p];
+        col[p] = t;
       }
-      const double t = col[s];
-      col[s] = col[p];
-      col[p] = t;
     }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < rows; i += blockDim.x) g[i] = col[i];
+}
+
+// Keeps its stream busy for about ns nanoseconds (at most 1000 naps of 100 ns).
+__global__ void head_start_kernel(int ns) {
+  for (int i = 0; i < min(ns / 100, 1000); ++i) __nanosleep(100);
 }
 
 // piv[i] = v for i in [lo, hi)
@@ -854,18 +870,16 @@ int laswp_forward(mo_ctx *ctx, View B, const int64_t *piv, int64_t npiv) {
   return MO_OK;
 }
 
-// the panel's interchanges on columns [c0, c1) of A through the move list of swap_map_kernel
+// the panel's interchanges on columns [c0, c1) of A through its move list
 int laswp_moves(mo_ctx *ctx, View A, int c0, int c1, const int *dst, const int *src,
-                const int *count, int max_moves) {
+                const int *count) {
   if (c1 <= c0) return MO_OK;
   const int nc = c1 - c0;
-  const size_t smem = (size_t)max_moves * 32 * sizeof(double);
-  if (int rc = mo_smem_attr((const void *)laswp_map_kernel, (int)smem)) return rc;
   ProfScope ps;
   prof_begin(ctx, ps, MO_PROF_LASWP);
-  laswp_map_kernel<<<(nc + 31) / 32, 256, smem, ctx->stream>>>(A.at(0, c0), A.ld, nc, dst, src,
-                                                               count);
-  prof_end(ctx, ps, 0.0, 16.0 * max_moves * (double)nc);
+  laswp_map_kernel<<<(nc + 31) / 32, 2 * MAX_PANEL_W, 0, ctx->stream>>>(A.at(0, c0), A.ld, nc, dst,
+                                                                        src, count);
+  prof_end(ctx, ps, 0.0, 16.0 * 2 * MAX_PANEL_W * (double)nc);
   MO_CUDA_TRY(cudaGetLastError());
   return MO_OK;
 }
@@ -901,7 +915,7 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
   const size_t sz_val = 2 * nblk * sizeof(double), sz_idx = 2 * nblk * sizeof(int);
   const size_t sz_row = (size_t)2 * nblk * W * sizeof(double), sz_rowj = 2 * W * sizeof(double);
   const size_t inv_bytes = 2 * 128 * 128 * sizeof(double);  // two panels' L11 inverses
-  const size_t sz_moves = 2 * (2 * MAX_PANEL_W) * sizeof(int) + 64;
+  const size_t sz_moves = 2 * (2 * (2 * MAX_PANEL_W) * sizeof(int) + 64);  // two panels'
   const size_t sz_ubuf = (size_t)kClL * kClSub * sizeof(double);
   const size_t total =
       inv_bytes + sz_ubuf + sz_val + sz_row + sz_rowj + sz_idx + 64 + 64 + sz_moves;
@@ -926,7 +940,18 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
   q += 16;
   int *abort_flag = (int *)q;
   q += 32;
-  int *mv_dst = (int *)q, *mv_src = mv_dst + 2 * MAX_PANEL_W, *mv_count = mv_src + 2 * MAX_PANEL_W;
+  // the moves of a pair's two panels; own: the panel's own columns are still to be put in order
+  struct Moves {
+    int *dst, *src, *count;
+    bool own;
+  } mv[2];
+  for (Moves &v : mv) {
+    v.dst = (int *)q;
+    v.src = v.dst + 2 * MAX_PANEL_W;
+    v.count = v.src + 2 * MAX_PANEL_W;
+    v.own = false;
+    q += 2 * (2 * MAX_PANEL_W) * sizeof(int) + 64;
+  }
 
   // rows up to which a panel may run in one cluster (the 16-CTA cluster is not portable: ask)
   int cl_rows = kClThreads * 8 * 4;
@@ -941,9 +966,10 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
     else
       cudaGetLastError();
   }
-  // one panel: factor A[k:m, k:k+b], then apply its interchanges to the other columns
-  auto panel = [&](int k, int b) -> int {
-    if (m - k <= cl_rows) {
+  // one panel: factor A[k:m, k:k+b] and list its interchanges
+  auto panel = [&](int k, int b, Moves &v) -> int {
+    v.own = m - k <= cl_rows;
+    if (v.own) {
       int rpt;
       const int ctas = cl_shape(m - k, &rpt);
       cudaLaunchConfig_t cfg;
@@ -955,11 +981,11 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
       double *Pd = A.at(k, k);
       int64_t pld = A.ld, *pv = piv + k, row0 = k;
       int pm = m - k, pw = b;
-      void *args[] = {&Pd, &pld, &pm, &pw, &pv, &row0, &ubuf, &mv_dst, &mv_src, &mv_count, &status};
+      void *args[] = {&Pd, &pld, &pm, &pw, &pv, &row0, &ubuf, &v.dst, &v.src, &v.count, &status};
       const cudaError_t e = cudaLaunchKernelExC(&cfg, cl_kernel(rpt), args);
       prof_end(ctx, ps, (double)(m - k) * b * b - (double)b * b * b / 3.0, 16.0 * (m - k) * b);
       MO_CUDA_TRY(e);
-      return laswp_moves(ctx, A, 0, n, mv_dst, mv_src, mv_count, 2 * b);
+      return MO_OK;
     }
     MO_CUDA_TRY(cudaMemsetAsync(sc.barrier, 0, 32, ctx->stream));  // barrier + abort flag
     View Pv = A.sub(k, k, m - k, b);
@@ -977,78 +1003,122 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
     MO_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)lu_panel_kernel, dim3(pblk),
                                             dim3(PANEL_THREADS), args, smem, ctx->stream));
     prof_end(ctx, ps, (double)pm * b * b - (double)b * b * b / 3.0, 16.0 * pm * b);
-    // interchanges on the columns left and right of the panel, as one move list
-    if (k > 0 || k + b < n) {
-      ProfScope pms;
-      prof_begin(ctx, pms, MO_PROF_LASWP);
-      if (m - k <= kSwapTableMax) {
-        const size_t tsm = (size_t)(m - k) * 5 + 2 * MAX_PANEL_W * sizeof(int) + 16;
-        int r2 = mo_smem_attr((const void *)swap_map_table_kernel, (int)tsm);
-        if (r2) return r2;
-        swap_map_table_kernel<<<1, 256, tsm, ctx->stream>>>(piv + k, b, k, m, mv_dst, mv_src,
-                                                            mv_count, status);
-      } else {
-        swap_map_kernel<<<1, 32, 0, ctx->stream>>>(piv + k, b, k, m, mv_dst, mv_src, mv_count,
-                                                   status);
-      }
-      prof_end(ctx, pms, 0.0, 8.0 * b);
-      MO_CUDA_TRY(cudaGetLastError());
+    ProfScope pms;
+    prof_begin(ctx, pms, MO_PROF_LASWP);
+    if (m - k <= kSwapTableMax) {
+      const size_t tsm = (size_t)(m - k) * 5 + 2 * MAX_PANEL_W * sizeof(int) + 16;
+      int r2 = mo_smem_attr((const void *)swap_map_table_kernel, (int)tsm);
+      if (r2) return r2;
+      swap_map_table_kernel<<<1, 256, tsm, ctx->stream>>>(piv + k, b, k, m, v.dst, v.src, v.count,
+                                                          status);
+    } else {
+      swap_map_kernel<<<1, 32, 0, ctx->stream>>>(piv + k, b, k, m, v.dst, v.src, v.count, status);
     }
-    int r2 = laswp_moves(ctx, A, 0, k, mv_dst, mv_src, mv_count, 2 * b);
-    if (!r2) r2 = laswp_moves(ctx, A, k + b, n, mv_dst, mv_src, mv_count, 2 * b);
+    prof_end(ctx, pms, 0.0, 8.0 * b);
+    MO_CUDA_TRY(cudaGetLastError());
+    return MO_OK;
+  };
+  // a panel's interchanges on the columns [c0, c1)
+  auto swap = [&](int k, int b, const Moves &v, int c0, int c1) -> int {
+    if (v.own) return laswp_moves(ctx, A, c0, c1, v.dst, v.src, v.count);
+    int r2 = laswp_moves(ctx, A, c0, std::min(c1, k), v.dst, v.src, v.count);
+    if (!r2) r2 = laswp_moves(ctx, A, std::max(c0, k + b), c1, v.dst, v.src, v.count);
     return r2;
   };
-  // Panels in pairs: the second panel's columns are brought up to date with the first
-  // (its U12 block and a (m - k2) x b1 x b0 update), the second is factored, and then the
-  // rows of the first two block rows right of the pair become U (two small products and
-  // one b1-row update between them) and the rest of the matrix takes ONE update with
-  // K = b0 + b1: the trailing matrix is read and written once per pair, not per panel.
+  // Panels in pairs: the first is factored, the second one's columns are brought up to date with
+  // it (U01 = inv0 A01, A[k2:m, P1] -= L[k2:m, P0] U01), the second is factored.  The
+  // interchanges are applied to the columns [c0, c1).
+  auto pair = [&](int k, int b0, int b1, int c0, int c1, const GemmOpts &o) -> int {
+    const int k2 = k + b0;
+    int r = panel(k, b0, mv[0]);
+    if (!r) r = swap(k, b0, mv[0], c0, c1);
+    if (!r && n > k2) r = trtri_blocks(ctx, A.sub(k, k, b0, b0), b0, false, true, true, inv);
+    if (r || b1 == 0) return r;
+    View U01 = A.sub(k, k2, b0, b1);
+    r = gemm_ex(ctx, U01, View{inv, b0, b0, 128}, false, U01, false, 1.0, 0.0, o);
+    if (!r)
+      r = gemm_ex(ctx, A.sub(k2, k2, m - k2, b1), A.sub(k2, k, m - k2, b0), false, U01, false, -1.0,
+                  1.0, o);
+    if (!r) r = panel(k2, b1, mv[1]);
+    if (!r) r = swap(k2, b1, mv[1], c0, c1);
+    if (!r && n > k2 + b1)
+      r = trtri_blocks(ctx, A.sub(k2, k2, b1, b1), b1, false, true, true, inv_b);
+    return r;
+  };
+  // Then the rows of the pair right of it become U (two small products and one b1-row update
+  // between them) and the rest of the matrix takes one update with K = b0 + b1, so the
+  // trailing matrix is read and written once per pair.
+  //
+  // Look-ahead: a pair is a chain of columns on one cluster (up to 16 SMs) and took as long as
+  // half of the update it waited for.  While the rest is wide, the next pair's columns are
+  // updated first and the pair is factored on the auxiliary stream, its interchanges applied
+  // to its own columns only, beside the update of the rest on the other SMs; the
+  // interchanges of the other columns follow.  The update is enqueued behind an event of the
+  // auxiliary stream that precedes the panel and a 5 us nap, so that the panel's cluster, which
+  // needs 16 free SMs in one part of the chip, is placed before the update fills it (without
+  // the nap the update mostly came first and the panel waited for its end).  Measured on B200,
+  // DecomposeLU: n = 16384 159.8 -> 130.1 ms, 8000 33.7 -> 26.6, 4000 10.8 -> 10.0, 3000 7.6 -> 7.3;
+  // below 1024 rows or columns of rest there is nothing to hide behind (n = 2000: no change).
+  constexpr int kAheadMin = 1024;
+  cudaStream_t s1 = nullptr;
+  bool ahead = false;  // the pair at k is being factored on the auxiliary stream
   for (int k = 0; k < mn; k += 2 * W) {
     const int b0 = min(W, mn - k);
-    if ((rc = panel(k, b0))) return rc;
     const int k2 = k + b0;
     const int b1 = k2 < mn ? min(W, mn - k2) : 0;
-    const int c_rest = n - k2 - b1;  // columns right of the pair
-    if (n - k2 > 0) {
-      if ((rc = trtri_blocks(ctx, A.sub(k, k, b0, b0), b0, false, true, true, inv))) return rc;
-    }
-    if (b1 == 0) {
-      // single last panel: U12 and the update of what is right of it
-      const int rest_c = n - k2;
-      if (rest_c > 0) {
-        View A12 = A.sub(k, k2, b0, rest_c);
-        if ((rc = gemm(ctx, A12, View{inv, b0, b0, 128}, false, A12, false, 1.0, 0.0))) return rc;
-        const int rest_r = m - k2;
-        if (rest_r > 0 && (rc = gemm(ctx, A.sub(k2, k2, rest_r, rest_c), A.sub(k2, k, rest_r, b0),
-                                     false, A12, false, -1.0, 1.0)))
-          return rc;
-      }
-      continue;
-    }
-    // the second panel's columns: U01 = inv0 A01, A[k2:m, P1] -= L[k2:m, P0] U01
-    {
-      View U01 = A.sub(k, k2, b0, b1);
-      if ((rc = gemm(ctx, U01, View{inv, b0, b0, 128}, false, U01, false, 1.0, 0.0))) return rc;
-      if ((rc = gemm(ctx, A.sub(k2, k2, m - k2, b1), A.sub(k2, k, m - k2, b0), false, U01, false,
-                     -1.0, 1.0)))
-        return rc;
-    }
-    if ((rc = panel(k2, b1))) return rc;
-    if (c_rest <= 0) continue;
     const int kc = k2 + b1;
-    if ((rc = trtri_blocks(ctx, A.sub(k2, k2, b1, b1), b1, false, true, true, inv_b))) return rc;
+    const int c_rest = n - kc;  // columns right of the pair
+    if (ahead) {
+      if ((rc = stream_wait(ctx, ctx->stream, s1, ctx->ev_join))) return rc;
+      if ((rc = swap(k, b0, mv[0], 0, k)) || (rc = swap(k, b0, mv[0], kc, n))) return rc;
+      if (b1 > 0 && ((rc = swap(k2, b1, mv[1], 0, k)) || (rc = swap(k2, b1, mv[1], kc, n)))) return rc;
+      ahead = false;
+    } else if ((rc = pair(k, b0, b1, 0, n, GemmOpts()))) {
+      return rc;
+    }
+    if (c_rest <= 0) continue;
     // rows k..k2 of the columns right of the pair: U0T = inv0 A0T
     View U0T = A.sub(k, kc, b0, c_rest);
     if ((rc = gemm(ctx, U0T, View{inv, b0, b0, 128}, false, U0T, false, 1.0, 0.0))) return rc;
-    // rows k2..kc: A1T -= L10 U0T, then U1T = inv1 A1T
-    View U1T = A.sub(k2, kc, b1, c_rest);
-    if ((rc = gemm(ctx, U1T, A.sub(k2, k, b1, b0), false, U0T, false, -1.0, 1.0))) return rc;
-    if ((rc = gemm(ctx, U1T, View{inv_b, b1, b1, 128}, false, U1T, false, 1.0, 0.0))) return rc;
+    if (b1 > 0) {
+      // rows k2..kc: A1T -= L10 U0T, then U1T = inv1 A1T
+      View U1T = A.sub(k2, kc, b1, c_rest);
+      if ((rc = gemm(ctx, U1T, A.sub(k2, k, b1, b0), false, U0T, false, -1.0, 1.0))) return rc;
+      if ((rc = gemm(ctx, U1T, View{inv_b, b1, b1, 128}, false, U1T, false, 1.0, 0.0))) return rc;
+    }
     // the rest: A[kc:m, kc:n] -= L[kc:m, k:kc] U[k:kc, kc:n]  (K = b0 + b1)
     const int rest_r = m - kc;
-    if (rest_r > 0 && (rc = gemm(ctx, A.sub(kc, kc, rest_r, c_rest), A.sub(kc, k, rest_r, b0 + b1),
-                                 false, A.sub(k, kc, b0 + b1, c_rest), false, -1.0, 1.0)))
-      return rc;
+    if (rest_r <= 0) continue;
+    const View Lp = A.sub(kc, k, rest_r, b0 + b1);
+    auto update = [&](int c0, int nc, const GemmOpts &o) {
+      return gemm_ex(ctx, A.sub(kc, c0, rest_r, nc), Lp, false, A.sub(k, c0, b0 + b1, nc), false, -1.0,
+                     1.0, o);
+    };
+    const int nb0 = kc < mn ? min(W, mn - kc) : 0;
+    const int nb1 = kc + nb0 < mn ? min(W, mn - kc - nb0) : 0;
+    const int nn = nb0 + nb1;
+    ahead = nb1 > 0 && rest_r <= cl_rows && c_rest - nn >= kAheadMin && rest_r >= kAheadMin;
+    if (!ahead) {
+      if ((rc = update(kc, c_rest, GemmOpts()))) return rc;
+      continue;
+    }
+    if ((rc = update(kc, nn, GemmOpts()))) return rc;
+    cudaStream_t s0 = ctx->stream;
+    if (!s1 && (rc = aux_stream(ctx, &s1))) return rc;
+    if ((rc = stream_wait(ctx, s1, s0, ctx->ev_fork))) return rc;
+    if ((rc = stream_wait(ctx, s0, s1, ctx->ev_join))) return rc;
+    {
+      StreamSwap sw(ctx, s1);
+      GemmOpts o;
+      o.stream_k = false;  // the stream-K scratch is the main stream's
+      o.max_ctas = kClMaxCtas;
+      if ((rc = pair(kc, nb0, nb1, kc, kc + nn, o))) return rc;
+    }
+    head_start_kernel<<<1, 1, 0, s0>>>(5000);
+    MO_CUDA_TRY(cudaGetLastError());
+    GemmOpts o;
+    o.max_ctas = ctx->sms - kClMaxCtas;
+    if ((rc = update(kc + nn, c_rest - nn, o))) return rc;
   }
   // The reference's blocked path (mlen > nb, nb != 0) leaves the pivot entries past
   // min(rows, cols) inside the last block equal to that block's start row (lu.go:216-219).
