@@ -1,0 +1,262 @@
+// The few-right-hand-side triangular solve in one thread-block cluster, for orders up to 2048
+// (included by trsm_few.cu, whose FewArgs it takes).
+//
+// A solve with few right-hand sides is a chain of diagonal blocks.  As CTAs that publish 64-row
+// steps through flags in L2 a 64-row step costs 4.6 us; here CTA c of a cluster of up to 16
+// owns the 128 rows of step c, keeps the inverse of its diagonal block in shared memory and
+// the next 128 x 128 block of op(A) in registers, adds up op(A) x for every step's x as it
+// arrives, and sends its own x to the later CTAs' shared memory (st.async onto an mbarrier per
+// step).  Each cluster takes up to 4 right-hand sides.
+// What bounds it: per 128 rows the exchange (about 800 cycles), 64 FMAs per thread and
+// right-hand side on the newest x, and the product with the inverse, whose 128 KB come from
+// shared memory.  Measured on B200, this kernel against the flag-passing one: n = 500, one
+// right-hand side 15 us (36 us); n = 1001, three 45 us (93 us).  SolveTrm as a whole, block
+// inverses (24 us) included: n = 2048, one right-hand side 170 -> 55 us, 16: 168 -> 89 us.
+#pragma once
+#include "cluster.cuh"
+
+namespace mo {
+namespace {
+
+constexpr int kTcThreads = 256, kTcBlock = 128, kTcMax = 16, kTcLd = kTcBlock + 1;
+
+template <int NR>
+struct TcSmem {
+  uint64_t bar[kTcMax];                              // arrival of step s's x
+  __align__(16) double x[kTcMax][NR * kTcBlock];     // x of the earlier steps, by right-hand side
+  __align__(16) double own[NR * kTcBlock];           // this CTA's x, and b before it
+  double part[NR * kTcBlock];
+  double inv[kTcBlock * kTcLd];                      // inv[k * kTcLd + i] = inverse(i, k)
+};
+
+template <typename TA, bool TRANS, int NR>
+__global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewArgs p) {
+  extern __shared__ __align__(16) unsigned char tc_raw[];
+  TcSmem<NR> &s = *reinterpret_cast<TcSmem<NR> *>(tc_raw);
+  if (p.skip && *(volatile const int *)p.skip) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nblk = (p.N + kTcBlock - 1) / kTcBlock;
+  const int c = blockIdx.x, rhs0 = blockIdx.y * NR, nr = min(NR, p.nrhs - rhs0);
+  const int r = tid & (kTcBlock - 1), h = tid >> 7;  // row, and which 64 of 128 columns
+  auto block = [&](int step) { return p.lower_eff ? step : nblk - 1 - step; };
+  const int rb = block(c), r0 = rb * kTcBlock;
+  const int nrow = c < nblk ? min(kTcBlock, p.N - r0) : 0;
+  const TA *A = static_cast<const TA *>(p.A);
+  // 64 elements of the 128 x 128 block of op(A) for step `step`: !TRANS: row r, columns 64 h + k at
+  // a[k]; TRANS: rows 16 warp + i, columns lane + 32 j at a[4 i + j] (contiguous along lanes)
+  TA a[64];
+  auto fetch = [&](int step) {
+    const int c0 = block(step) * kTcBlock, nc = min(kTcBlock, p.N - c0);
+    if constexpr (!TRANS) {
+      const TA *src = A + r0 + r + (int64_t)(c0 + 64 * h) * p.lda;
+#pragma unroll
+      for (int k = 0; k < 64; ++k) a[k] = r < nrow && 64 * h + k < nc ? src[k * p.lda] : TA(0);
+    } else {
+      const TA *src = A + c0 + lane + (int64_t)(r0 + 16 * warp) * p.lda;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          a[4 * i + j] =
+              16 * warp + i < nrow && lane + 32 * j < nc ? src[i * p.lda + 32 * j] : TA(0);
+    }
+  };
+  if (c > 0 && c < nblk) fetch(0);
+  if (tid == 0) {
+    for (int t = 0; t < kTcMax; ++t) mbar_init(&s.bar[t], 1);
+    fence_barrier_init();
+    for (int t = 0; t < c && c < nblk; ++t)
+      mbar_arrive_expect_tx(&s.bar[t], (uint32_t)(NR * kTcBlock * sizeof(double)));
+  }
+  if (c < nblk) {
+    const double *iv = p.inv + (size_t)rb * kTcBlock * kTcBlock;
+#pragma unroll 16
+    for (int e = tid; e < kTcBlock * kTcBlock; e += kTcThreads) {
+      const int u = e & (kTcBlock - 1), w = e >> 7;
+      const double v = u < nrow && w < nrow ? iv[e] : 0.0;
+      if (p.inv_t) s.inv[u * kTcLd + w] = v;
+      else s.inv[w * kTcLd + u] = v;
+    }
+  }
+  cl_sync();  // every CTA's barriers are armed before any x is sent
+  double acc[NR];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) acc[q] = 0.0;
+  double sum[16 * NR];  // TRANS: this lane's part of the rows 16 warp + i
+  if constexpr (TRANS) {
+#pragma unroll
+    for (int i = 0; i < 16 * NR; ++i) sum[i] = 0.0;
+  }
+  if (c < nblk) {
+    for (int t = 0; t < c; ++t) {
+      // (a wait that runs out is recorded; the kernel goes on with what it holds)
+      mbar_wait(&s.bar[t], 0, p.status);
+      if constexpr (!TRANS) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          const double2 *x = reinterpret_cast<const double2 *>(s.x[t] + q * kTcBlock + 64 * h);
+          double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+#pragma unroll
+          for (int k = 0; k < 64; k += 4) {
+            const double2 xa = x[k / 2], xb = x[k / 2 + 1];
+            v0 = fma((double)a[k], xa.x, v0);
+            v1 = fma((double)a[k + 1], xa.y, v1);
+            v2 = fma((double)a[k + 2], xb.x, v2);
+            v3 = fma((double)a[k + 3], xb.y, v3);
+          }
+          acc[q] += (v0 + v1) + (v2 + v3);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          double x[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[j] = s.x[t][q * kTcBlock + lane + 32 * j];
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              sum[16 * q + i] = fma((double)a[4 * i + j], x[j], sum[16 * q + i]);
+        }
+      }
+      if (t + 1 < c) fetch(t + 1);
+    }
+    // b = alpha B - sum, complete in s.own
+    if constexpr (!TRANS) {
+      if (h == 1) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = acc[q];
+      }
+    } else {
+      // 16 rows over 32 lanes: lane l ends with row l / 2 of the warp's
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+#pragma unroll
+        for (int o = 16; o > 1; o >>= 1) {
+#pragma unroll
+          for (int k = 0; k < o / 2; ++k) {
+            const bool up = lane & o;
+            const double give = up ? sum[16 * q + k] : sum[16 * q + k + o / 2];
+            const double keep = up ? sum[16 * q + k + o / 2] : sum[16 * q + k];
+            sum[16 * q + k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        const double v = sum[16 * q] + __shfl_xor_sync(0xffffffffu, sum[16 * q], 1);
+        if (!(lane & 1)) s.part[q * kTcBlock + 16 * warp + (lane >> 1)] = v;
+      }
+    }
+    __syncthreads();
+    if (h == 0) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const double b = r < nrow && q < nr ? p.alpha * p.B[(int64_t)(r0 + r) * p.brs +
+                                                           (int64_t)(rhs0 + q) * p.bcs]
+                                            : 0.0;
+        s.own[q * kTcBlock + r] = b - (TRANS ? s.part[q * kTcBlock + r]
+                                             : acc[q] + s.part[q * kTcBlock + r]);
+      }
+    }
+    __syncthreads();
+    // x = inverse b
+    double x[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) x[q] = 0.0;
+    const double *iv = s.inv + 64 * h * kTcLd + r;
+    // (the inverse's 64 x 64 block of zeros is left out: an infinity in b stays on its side)
+    if (h == (r >> 6) || (h == 0) == (p.lower_eff != 0)) {
+#pragma unroll 16
+      for (int k = 0; k < 64; ++k) {
+        const double v = iv[k * kTcLd];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) x[q] = fma(v, s.own[q * kTcBlock + 64 * h + k], x[q]);
+      }
+    }
+    if (h == 1) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
+    }
+    __syncthreads();
+    if (h == 0) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const double v = r < nrow ? x[q] + s.part[q * kTcBlock + r] : 0.0;
+        s.own[q * kTcBlock + r] = v;
+        if (r < nrow && q < nr)
+          p.B[(int64_t)(r0 + r) * p.brs + (int64_t)(rhs0 + q) * p.bcs] = v;
+      }
+    }
+    __syncthreads();
+    // to the later CTAs, a warp per CTA
+    for (int d = c + 1 + warp; d < nblk; d += kTcThreads / 32) {
+      const uint32_t to = cl_map(s.x[c], d), mb = cl_map(&s.bar[c], d);
+      const double2 *src = reinterpret_cast<const double2 *>(s.own);
+#pragma unroll
+      for (int e = lane; e < NR * kTcBlock / 2; e += 32) {
+        const double2 v = src[e];
+        asm volatile(
+            "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
+                to + 16 * e),
+            "d"(v.x), "d"(v.y), "r"(mb)
+            : "memory");
+      }
+    }
+  }
+  cl_sync();  // no CTA leaves while another may still write into its memory
+}
+
+template <typename TA, bool TRANS, int NR>
+int tc_launch(mo_ctx *ctx, const FewArgs &p, int ctas, int groups) {
+  const void *fn = (const void *)trsm_cluster_kernel<TA, TRANS, NR>;
+  if (int rc = mo_smem_attr(fn, (int)sizeof(TcSmem<NR>))) return rc;
+  MO_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas, groups);
+  cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = sizeof(TcSmem<NR>);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {(unsigned)ctas, 1, 1};
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (ctas > 8) {  // not portable: ask
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, trsm_cluster_kernel<TA, TRANS, NR>, &cfg) != cudaSuccess ||
+        clusters < 1) {
+      cudaGetLastError();
+      return 1;
+    }
+  }
+  void *args[] = {const_cast<FewArgs *>(&p)};
+  ProfScope ps;
+  prof_begin(ctx, ps, sizeof(TA) == 4 ? MO_PROF_IR : MO_PROF_GEMM);
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+  prof_end(ctx, ps, (double)p.N * p.N * p.nrhs,
+           sizeof(TA) * (double)p.N * p.N / 2 + 8.0 * 2.0 * p.N * p.nrhs);
+  MO_CUDA_TRY(e);
+  return MO_OK;
+}
+
+// MO_OK, an error, or 1: not for the cluster.  A cluster holds 16 blocks of 128; more CTAs than
+// the chip runs at a time (one of 16 CTAs per 18 SMs or so) go in a second wave: measured at 128
+// CTAs, n = 2048 and 32 right-hand sides, 158 us (flag-passing 220 us), while past it 64
+// right-hand sides would take two more
+template <typename TA>
+int tc_run(mo_ctx *ctx, const FewArgs &p) {
+  const int nblk = (p.N + kTcBlock - 1) / kTcBlock;
+  if (nblk > kTcMax) return 1;
+  int ctas = 1;
+  while (ctas < nblk) ctas *= 2;
+  const int per = p.nrhs > 2 ? 4 : p.nrhs, groups = (p.nrhs + per - 1) / per;
+  if (groups * ctas > 128) return 1;
+  if (p.trans)
+    return per == 1   ? tc_launch<TA, true, 1>(ctx, p, ctas, groups)
+           : per == 2 ? tc_launch<TA, true, 2>(ctx, p, ctas, groups)
+                      : tc_launch<TA, true, 4>(ctx, p, ctas, groups);
+  return per == 1   ? tc_launch<TA, false, 1>(ctx, p, ctas, groups)
+         : per == 2 ? tc_launch<TA, false, 2>(ctx, p, ctas, groups)
+                    : tc_launch<TA, false, 4>(ctx, p, ctas, groups);
+}
+
+}  // namespace
+}  // namespace mo

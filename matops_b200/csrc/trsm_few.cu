@@ -566,6 +566,14 @@ int launch_pair(mo_ctx *ctx, FewArgs &p) {
   return MO_OK;
 }
 
+}  // namespace
+}  // namespace mo
+
+#include "trsm_cluster.cuh"
+
+namespace mo {
+namespace {
+
 // flags -> (B strides, effective transposition and sweep direction) and the launch
 int few_run(mo_ctx *ctx, View B, const void *A, bool a32, int64_t lda, int N, int flags,
             double alpha, const double *inv, bool inv_t, int *flag_buf,
@@ -604,6 +612,11 @@ int few_run(mo_ctx *ctx, View B, const void *A, bool a32, int64_t lda, int N, in
   p.status = reinterpret_cast<int *>(ctx->d_status);
   p.spin_limit = ctx->spin_limit;
   p.skip = skip;
+  // up to 16 blocks of 128: one cluster per 4 right-hand sides
+  {
+    const int rc = a32 ? tc_run<float>(ctx, p) : tc_run<double>(ctx, p);
+    if (rc <= 0) return rc;
+  }
   // more than MO_FEW_GROUP columns: groups solved side by side by separate CTA sets, so
   // the per-step work on the dependency chain is that of one group
   const bool pair = a32 && p.nblk >= 4;
