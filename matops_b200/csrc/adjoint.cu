@@ -562,8 +562,7 @@ extern "C" int mo_solve_chol_adjoint(mo_ctx *ctx, mo_matrix Lm, mo_matrix Xm, mo
   if (flags & MO_UPPER) return MO_EINVAL;
   if (L.rows == 0 || X.cols == 0) return MO_OK;
   // Bbar = (L L^T)^-1 Xbar, as SolveCHOL LOWER (chol.go:151-153)
-  if ((rc = trsm(ctx, XB, L, MO_LOWER, 1.0))) return rc;
-  if ((rc = trsm(ctx, XB, L, MO_LOWER | MO_TRANSA, 1.0))) return rc;
+  if ((rc = trsm_pair(ctx, XB, L, MO_LOWER))) return rc;
   // Abar -= (Bbar X^T + X Bbar^T) / 2
   if ((rc = gemm(ctx, G, XB, false, X, true, -0.5, 1.0))) return rc;
   return gemm(ctx, G, X, false, XB, true, -0.5, 1.0);

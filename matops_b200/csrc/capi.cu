@@ -402,8 +402,8 @@ int mo_rank_update_sym(mo_ctx *ctx, mo_matrix Cm, mo_matrix Am, double alpha, do
   return mo::syrk(ctx, C, A, ta, up, alpha, beta, bb);
 }
 
-// mmult.go:388-422
-int mo_solve_trm(mo_ctx *ctx, mo_matrix Bm, mo_matrix Am, double alpha, int flags) {
+// mmult.go:388-422 (pair: then the same with the other transposition)
+static int solve_trm(mo_ctx *ctx, mo_matrix Bm, mo_matrix Am, double alpha, int flags, bool pair) {
   int rc = mo::enter(ctx);
   if (rc) return rc;
   View B, A;
@@ -430,7 +430,12 @@ int mo_solve_trm(mo_ctx *ctx, mo_matrix Bm, mo_matrix Am, double alpha, int flag
   if (N == 0 || (right ? B.rows : B.cols) == 0) return MO_OK;
   if (A.rows < N || (right ? B.cols : B.rows) < N) return MO_EABSIZE;
   View Bn = right ? B.sub(0, 0, B.rows, N) : B.sub(0, 0, N, B.cols);
-  return mo::trsm(ctx, Bn, A.sub(0, 0, N, N), flags, alpha);
+  const View An = A.sub(0, 0, N, N);
+  return pair ? mo::trsm_pair(ctx, Bn, An, flags) : mo::trsm(ctx, Bn, An, flags, alpha);
+}
+
+int mo_solve_trm(mo_ctx *ctx, mo_matrix Bm, mo_matrix Am, double alpha, int flags) {
+  return solve_trm(ctx, Bm, Am, alpha, flags, false);
 }
 
 // chol.go:116-127
@@ -462,17 +467,8 @@ int mo_decompose_chol(mo_ctx *ctx, mo_matrix Am, int flags, int nb, double *bad_
 
 // chol.go:147-158
 int mo_solve_chol(mo_ctx *ctx, mo_matrix Bm, mo_matrix Am, int flags) {
-  int rc;
-  if (flags & MO_UPPER) {
-    rc = mo_solve_trm(ctx, Bm, Am, 1.0, MO_UPPER | MO_TRANSA);
-    if (!rc) rc = mo_solve_trm(ctx, Bm, Am, 1.0, MO_UPPER);
-    return rc;
-  }
-  if (flags & MO_LOWER) {
-    rc = mo_solve_trm(ctx, Bm, Am, 1.0, MO_LOWER);
-    if (!rc) rc = mo_solve_trm(ctx, Bm, Am, 1.0, MO_LOWER | MO_TRANSA);
-    return rc;
-  }
+  if (flags & MO_UPPER) return solve_trm(ctx, Bm, Am, 1.0, MO_UPPER | MO_TRANSA, true);
+  if (flags & MO_LOWER) return solve_trm(ctx, Bm, Am, 1.0, MO_LOWER, true);
   return MO_OK;
 }
 

@@ -665,13 +665,7 @@ int fp64_solve(mo_ctx *ctx, const View &A, bool upper, const View &X, const doub
       break;
     }
     vcopy_kernel<<<vgrid(n, X.cols), 256, 0, ctx->stream>>>(X.d, X.ld, b, n, n, X.cols);
-    if (upper) {
-      rc = trsm(ctx, X, T, MO_UPPER | MO_TRANSA, 1.0);
-      if (!rc) rc = trsm(ctx, X, T, MO_UPPER, 1.0);
-    } else {
-      rc = trsm(ctx, X, T, MO_LOWER, 1.0);
-      if (!rc) rc = trsm(ctx, X, T, MO_LOWER | MO_TRANSA, 1.0);
-    }
+    rc = trsm_pair(ctx, X, T, upper ? MO_UPPER | MO_TRANSA : MO_LOWER);
     if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = MO_ECUDA;
   } while (false);
   cudaStreamSynchronize(ctx->stream);

@@ -55,9 +55,12 @@ int trtri_blocks(mo_ctx *ctx, View A, int N, bool trans, bool lower_eff, bool un
   return MO_OK;
 }
 
-int trsm_few(mo_ctx *ctx, View B, View A, int flags, double alpha, double *inv, int *flag_buf);
+int trsm_few(mo_ctx *ctx, View B, View A, int flags, double alpha, double *inv, int *flag_buf,
+             bool pair);
 
-int trsm(mo_ctx *ctx, View B, View A, int flags, double alpha) {
+namespace {
+
+int trsm_sweeps(mo_ctx *ctx, View B, View A, int flags, double alpha, bool pair) {
   const int N = A.cols;
   const int nrhs = (flags & MO_RIGHT) ? B.rows : B.cols;
   if (N == 0 || nrhs == 0) return MO_OK;
@@ -71,8 +74,20 @@ int trsm(mo_ctx *ctx, View B, View A, int flags, double alpha) {
   // few right-hand sides: one cooperative launch instead of a sweep of 2*nblk GEMMs
   if (nblk > 1 && nrhs <= 64)
     return trsm_few(ctx, B, A, flags, alpha, inv,
-                    reinterpret_cast<int *>(reinterpret_cast<char *>(inv) + inv_bytes));
-  return trsm_with_scratch(ctx, B, A, flags, alpha, inv);
+                    reinterpret_cast<int *>(reinterpret_cast<char *>(inv) + inv_bytes), pair);
+  rc = trsm_with_scratch(ctx, B, A, flags, alpha, inv);
+  if (!rc && pair) rc = trsm_with_scratch(ctx, B, A, flags ^ MO_TRANSA, 1.0, inv);
+  return rc;
+}
+
+}  // namespace
+
+int trsm(mo_ctx *ctx, View B, View A, int flags, double alpha) {
+  return trsm_sweeps(ctx, B, A, flags, alpha, false);
+}
+
+int trsm_pair(mo_ctx *ctx, View B, View A, int flags) {
+  return trsm_sweeps(ctx, B, A, flags, 1.0, true);
 }
 
 // The sweep of trsm() with the caller's scratch for the inverted diagonal blocks

@@ -44,3 +44,21 @@ def test_sizes(gpu, rng, n, flags, nrhs):
 def test_right_hand_sides(gpu, rng, nrhs, side, flags):
     _solve(gpu, rng, 300, nrhs, side | flags, alpha=-1.5)
     _solve(gpu, rng, 1300, nrhs, side | flags)
+
+
+@pytest.mark.parametrize("n", [128, 129, 700, 2049])
+@pytest.mark.parametrize("flags", [LO, UP])
+@pytest.mark.parametrize("nrhs", [1, 5, 65])
+def test_cholesky_sweeps_are_the_two_solves(gpu, rng, n, flags, nrhs):
+    # SolveCHOL forms the block inverses once for both sweeps: the same operations, bit for bit
+    A = gpu.matrix(n, n)
+    import torch
+    A.copy_(torch.from_numpy(rng.uniform(-1, 1, (n, n)) / n + 2.0 * np.eye(n)))
+    B, C = gpu.matrix(n, nrhs), gpu.matrix(n, nrhs)
+    B.copy_(torch.from_numpy(rng.uniform(-1, 1, (n, nrhs))))
+    C.copy_(B)
+    gpu.SolveCHOL(B, A, flags)
+    for f in ((flags, flags | TA) if flags == LO else (flags | TA, flags)):
+        assert gpu.SolveTrm(C, A, 1.0, LEFT | f) is None
+    assert gpu.Sync() == 0
+    assert torch.equal(B, C)
