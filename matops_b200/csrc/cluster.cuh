@@ -16,20 +16,20 @@ __device__ __forceinline__ void cl_sync() {
 }
 
 // PIECES x 16 bytes at `src` (this CTA's shared memory, 16-byte aligned) to the same place `dst`
-// of every CTA of the cluster (at most 16), the bytes counted on that CTA's barrier `bar`: the
-// calling warp's lane pair (2 c, 2 c + 1) writes CTA c's copy.  (Plain remote stores need a
+// of every CTA of the cluster (at most 32 / LANES), the bytes counted on that CTA's barrier `bar`:
+// lanes LANES c, ... of the calling warp write CTA c's copy.  (Plain remote stores need a
 // cluster barrier with release semantics, which also waits for the panel's global stores: 1330
 // cycles a column of the LU panel, 850 this way.)
-template <int PIECES>
+template <int PIECES, int LANES = 2>
 __device__ __forceinline__ void cl_send(void *dst, const void *src, uint64_t *bar, int lane,
                                         int nctas) {
-  const int c = lane >> 1;
+  const int c = lane / LANES;
   if (c >= nctas) return;
   const uint32_t to = cl_map(dst, c), mb = cl_map(bar, c);
   const double2 *s = reinterpret_cast<const double2 *>(src);
 #pragma unroll
-  for (int i = 0; i < (PIECES + 1) / 2; ++i) {
-    const int p = 2 * i + (lane & 1);
+  for (int i = 0; i < (PIECES + LANES - 1) / LANES; ++i) {
+    const int p = LANES * i + lane % LANES;
     if (p < PIECES) {
       const double2 v = s[p];
       asm volatile(

@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(PANEL_THREADS)
 // the exchange; the triangle of U and the left-looking products take the other third.
 constexpr int kClThreads = 256, kClWarps = kClThreads / 32, kClSub = 16, kClMaxCtas = 16;
 constexpr int kClMaxRows = kClThreads * kClMaxCtas * 4;
+constexpr int kClByWarp = 4, kClCands = kClByWarp * kClWarps;  // (one lane per candidate)
 constexpr int kClL = MAX_PANEL_W - kClSub;  // rows of U that a later sub-panel needs
 constexpr int kClLd = kClL + 2;  // a row of L^T (16-byte aligned, 4 banks from the next)
 
@@ -280,9 +281,9 @@ struct __align__(16) ClRow {
 struct ClSmem {
   uint64_t bar[2];            // arrival of a column's packets, by column parity
   uint64_t pad[2];
-  ClRow recv[2][kClMaxCtas];  // one candidate per CTA, double-buffered by column
+  ClRow recv[2][kClCands];    // a candidate per CTA or per warp, double-buffered by column
   ClRow rowj[2];              // the row at the diagonal
-  ClRow own;                  // this CTA's candidate, gathered for sending
+  ClRow own[kClWarps];        // this CTA's (own[0]) or each warp's candidate, for sending
   ClRow ownj;                 // (CTA 0) the diagonal row, gathered for sending
   unsigned red_hi[2][kClWarps], red_lo[2][kClWarps];
   int red_idx[2][kClWarps];
@@ -303,7 +304,10 @@ __device__ __forceinline__ void cl_argmax(unsigned &hi, unsigned &lo, int &idx) 
   lo = l;
 }
 
-template <int RPT>
+// BY_WARP (at most kClByWarp CTAs): every warp sends its own candidate to every CTA, which spares
+// the second argmax level and a block barrier per column; more CTAs would receive more
+// candidates than a warp has lanes, and many times the bytes, so there a CTA sends one.
+template <int RPT, bool BY_WARP>
 __global__ void __launch_bounds__(kClThreads, 1)
     lu_cluster_panel_kernel(double *P, int64_t ld, int m, int W, int64_t *piv, int64_t row0,
                             double *ubuf, int *mv_dst, int *mv_src, int *mv_count,
@@ -473,9 +477,33 @@ __global__ void __launch_bounds__(kClThreads, 1)
       const int jc = j0 + c, par = jc & 1;
       // this column's packets: one candidate per CTA and the diagonal row
       if (nctas > 1 && tid == 0)
-        mbar_arrive_expect_tx(&s.bar[par], (uint32_t)((nctas + 1) * sizeof(ClRow)));
+        mbar_arrive_expect_tx(&s.bar[par],
+                              (uint32_t)((nctas * (BY_WARP ? kClWarps : 1) + 1) * sizeof(ClRow)));
       cl_argmax(hi, lo, idx);
-      if (lane == 0) {
+      // the candidate row, from its owner's registers
+      auto gather = [&](ClRow &to) {
+        if (idx == INT_MAX && lane == 0) {  // no row left in this CTA (warp)
+          to.hi = to.lo = 0u;
+          to.idx = INT_MAX;
+        }
+#pragma unroll
+        for (int q = 0; q < RPT; ++q)
+          if (rbase + kClThreads * q == idx) {
+#pragma unroll
+            for (int k = 0; k < kClSub; ++k) to.x[k] = x[q][k];
+            to.hi = hi;
+            to.lo = lo;
+            to.idx = idx;
+            to.phys = phys[q];
+          }
+        __syncwarp();
+      };
+      if constexpr (BY_WARP) {
+        gather(nctas > 1 ? s.own[warp] : s.recv[par][warp]);
+        if (nctas > 1)
+          cl_send<9, 32 / kClByWarp>(&s.recv[par][cta * kClWarps + warp], &s.own[warp],
+                                     &s.bar[par], lane, nctas);
+      } else if (lane == 0) {
         s.red_hi[par][warp] = hi;
         s.red_lo[par][warp] = lo;
         s.red_idx[par][warp] = idx;
@@ -491,56 +519,41 @@ __global__ void __launch_bounds__(kClThreads, 1)
         __syncwarp();
         if (nctas > 1) cl_send<9>(&s.rowj[par], &s.ownj, &s.bar[par], lane, nctas);
       }
-      __syncthreads();
-      hi = s.red_hi[par][lane & (kClWarps - 1)];
-      lo = s.red_lo[par][lane & (kClWarps - 1)];
-      idx = s.red_idx[par][lane & (kClWarps - 1)];
-      cl_argmax(hi, lo, idx);
-      // this CTA's candidate, from its owner's registers to every CTA
-      if (warp == (idx == INT_MAX ? 0 : (idx & (kClThreads - 1)) >> 5)) {
-        ClRow &to = nctas > 1 ? s.own : s.recv[par][0];
-        if (idx == INT_MAX && lane == 0) {  // no row left in this CTA
-          to.hi = to.lo = 0u;
-          to.idx = INT_MAX;
+      if constexpr (!BY_WARP) {
+        __syncthreads();
+        hi = s.red_hi[par][lane & (kClWarps - 1)];
+        lo = s.red_lo[par][lane & (kClWarps - 1)];
+        idx = s.red_idx[par][lane & (kClWarps - 1)];
+        cl_argmax(hi, lo, idx);
+        // this CTA's candidate to every CTA
+        if (warp == (idx == INT_MAX ? 0 : (idx & (kClThreads - 1)) >> 5)) {
+          gather(s.own[0]);
+          cl_send<9>(&s.recv[par][cta], &s.own[0], &s.bar[par], lane, nctas);
         }
-#pragma unroll
-        for (int q = 0; q < RPT; ++q)
-          if (rbase + kClThreads * q == idx) {
-#pragma unroll
-            for (int k = 0; k < kClSub; ++k) to.x[k] = x[q][k];
-            to.hi = hi;
-            to.lo = lo;
-            to.idx = idx;
-            to.phys = phys[q];
-          }
-        __syncwarp();
-        if (nctas > 1) cl_send<9>(&s.recv[par][cta], &s.own, &s.bar[par], lane, nctas);
       }
       // every warp picks the pivot: largest key, lowest row
-      if (nctas > 1) {
-        // (a wait that runs out is recorded; the kernel goes on with what it holds)
-        mbar_wait(&s.bar[par], (jc >> 1) & 1, status);
-        const ClRow &cand = s.recv[par][lane < nctas ? lane : 0];
-        hi = cand.hi;
-        lo = cand.lo;
-        idx = cand.idx;
-        cl_argmax(hi, lo, idx);
-      } else {
-        __syncthreads();
-      }
+      // (a wait that runs out is recorded; the kernel goes on with what it holds)
+      if (nctas > 1) mbar_wait(&s.bar[par], (jc >> 1) & 1, status);
+      else __syncthreads();
+      const int cands = BY_WARP ? nctas * kClWarps : nctas;
+      const ClRow &cand = s.recv[par][lane < cands ? lane : 0];
+      hi = cand.hi;
+      lo = cand.lo;
+      idx = cand.idx;
+      cl_argmax(hi, lo, idx);
       const int p = min(max(idx, jc), m - 1);  // (idx itself, unless a wait ran out)
-      const ClRow &pr = s.recv[par][p / (kClThreads * RPT)];
+      const ClRow &pr = s.recv[par][p / (BY_WARP ? 32 : kClThreads * RPT)];
+      if (cta == 0 && warp == kClWarps - 1) {  // the U row, and the pivot
+        if (lane < w - c)
+          P[min(max(pr.phys, 0), m - 1) + (int64_t)(jc + lane) * ld] = pr.x[lane];
+        if (lane == 0) piv[jc] = row0 + p;
+      }
       double u[kClSub];
 #pragma unroll
       for (int k = 0; k < kClSub / 2; ++k) {
         const double2 v = reinterpret_cast<const double2 *>(pr.x)[k];
         u[2 * k] = v.x;
         u[2 * k + 1] = v.y;
-      }
-      if (cta == 0 && warp == kClWarps - 1) {  // the U row, and the pivot
-        if (lane < w - c)
-          P[min(max(pr.phys, 0), m - 1) + (int64_t)(jc + lane) * ld] = pr.x[lane];
-        if (lane == 0) piv[jc] = row0 + p;
       }
       if (p != jc && (warp == ((p & (kClThreads - 1)) >> 5) || warp == jc / 32)) {
 #pragma unroll
@@ -601,15 +614,16 @@ inline int cl_shape(int m, int *rpt) {
   return c;
 }
 
-const void *cl_kernel(int rpt) {
-  return rpt == 1   ? (const void *)lu_cluster_panel_kernel<1>
-         : rpt == 2 ? (const void *)lu_cluster_panel_kernel<2>
-                    : (const void *)lu_cluster_panel_kernel<4>;
+const void *cl_kernel(int ctas, int rpt) {
+  return ctas <= kClByWarp ? (const void *)lu_cluster_panel_kernel<1, true>
+         : rpt == 1        ? (const void *)lu_cluster_panel_kernel<1, false>
+         : rpt == 2        ? (const void *)lu_cluster_panel_kernel<2, false>
+                           : (const void *)lu_cluster_panel_kernel<4, false>;
 }
 
 int cl_config(int ctas, int rpt, cudaStream_t st, cudaLaunchConfig_t *cfg,
               cudaLaunchAttribute *attr) {
-  const void *fn = cl_kernel(rpt);
+  const void *fn = cl_kernel(ctas, rpt);
   if (int rc = mo_smem_attr(fn, (int)sizeof(ClSmem))) return rc;
   MO_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   *cfg = cudaLaunchConfig_t{};
@@ -960,7 +974,7 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
     cudaLaunchAttribute attr;
     int clusters = 0;
     if ((rc = cl_config(kClMaxCtas, 4, ctx->stream, &cfg, &attr))) return rc;
-    if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(4), &cfg) == cudaSuccess &&
+    if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(kClMaxCtas, 4), &cfg) == cudaSuccess &&
         clusters > 0)
       cl_rows = kClMaxRows;
     else
@@ -982,7 +996,7 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
       int64_t pld = A.ld, *pv = piv + k, row0 = k;
       int pm = m - k, pw = b;
       void *args[] = {&Pd, &pld, &pm, &pw, &pv, &row0, &ubuf, &v.dst, &v.src, &v.count, &status};
-      const cudaError_t e = cudaLaunchKernelExC(&cfg, cl_kernel(rpt), args);
+      const cudaError_t e = cudaLaunchKernelExC(&cfg, cl_kernel(ctas, rpt), args);
       prof_end(ctx, ps, (double)(m - k) * b * b - (double)b * b * b / 3.0, 16.0 * (m - k) * b);
       MO_CUDA_TRY(e);
       return MO_OK;
