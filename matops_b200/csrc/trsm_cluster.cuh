@@ -29,6 +29,25 @@ struct TcSmem {
   double inv[kTcBlock * kTcLd];                      // inv[k * kTcLd + i] = inverse(i, k)
 };
 
+// The wait for a step's x: with fewer polls than usual allowed (mo_set_spin_limit) one that runs
+// out is recorded, and the x still waited for, since it lands in this CTA's memory either way.
+__device__ __forceinline__ void tc_wait(uint64_t *bar, const FewArgs &p) {
+  if (p.spin_limit < MO_SPIN_LIMIT) {
+    for (uint32_t it = 0; it <= p.spin_limit; ++it) {
+      uint32_t done;
+      asm volatile(
+          "{\n\t.reg .pred q;\n\tmbarrier.test_wait.parity.shared::cta.b64 q, [%1], 0;\n\t"
+          "selp.u32 %0, 1, 0, q;\n\t}"
+          : "=r"(done)
+          : "r"(smem_u32(bar))
+          : "memory");
+      if (done) return;
+    }
+    set_status(p.status, MO_EDEVTIMEOUT);
+  }
+  mbar_wait(bar, 0, p.status);
+}
+
 template <typename TA, bool TRANS, int NR>
 __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewArgs p) {
   extern __shared__ __align__(16) unsigned char tc_raw[];
@@ -89,8 +108,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
   }
   if (c < nblk) {
     for (int t = 0; t < c; ++t) {
-      // (a wait that runs out is recorded; the kernel goes on with what it holds)
-      mbar_wait(&s.bar[t], 0, p.status);
+      tc_wait(&s.bar[t], p);
       if constexpr (!TRANS) {
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -237,10 +255,8 @@ int tc_launch(mo_ctx *ctx, const FewArgs &p, int ctas, int groups) {
   return MO_OK;
 }
 
-// MO_OK, an error, or 1: not for the cluster.  A cluster holds 16 blocks of 128; more CTAs than
-// the chip runs at a time (one of 16 CTAs per 18 SMs or so) go in a second wave: measured at 128
-// CTAs, n = 2048 and 32 right-hand sides, 158 us (flag-passing 220 us), while past it 64
-// right-hand sides would take two more
+// MO_OK, an error, or 1: not for the cluster (more than 16 blocks of 128, or more than 128 CTAs,
+// which would run in several waves; the FP64 callers cut their blocks to fit, few_sweep)
 template <typename TA>
 int tc_run(mo_ctx *ctx, const FewArgs &p) {
   const int nblk = (p.N + kTcBlock - 1) / kTcBlock;

@@ -1,7 +1,7 @@
-"""SolveTrm with few right-hand sides up to order 2048 (one thread-block cluster, 128 rows per CTA,
-up to 4 right-hand sides each) at the edges of its blocks and cluster sizes, all sides,
-triangles and transpositions, with odd leading dimensions; bound 100 n eps relative, as in
-the parity tests of SolveTrm.  Sizes past it take the flag-passing kernel."""
+"""SolveTrm with few right-hand sides: up to order 2048 one thread-block cluster per 4 of them
+(128 rows per CTA), above by blocks of 512, 1024 or 2048; at the edges of the blocks and cluster
+sizes, all sides, triangles and transpositions, with odd leading dimensions; bound 100 n eps
+relative, as in the parity tests of SolveTrm."""
 import numpy as np
 import pytest
 
@@ -62,3 +62,12 @@ def test_cholesky_sweeps_are_the_two_solves(gpu, rng, n, flags, nrhs):
         assert gpu.SolveTrm(C, A, 1.0, LEFT | f) is None
     assert gpu.Sync() == 0
     assert torch.equal(B, C)
+
+
+@pytest.mark.parametrize("n,nrhs", [(1025, 17), (2048, 64), (2177, 33), (4097, 1), (4200, 20),
+                                    (513, 49)])
+@pytest.mark.parametrize("side", [LEFT, RIGHT])
+@pytest.mark.parametrize("flags", [LO, UP | UNIT, LO | TA, UP | TA])
+def test_blocks(gpu, rng, n, nrhs, side, flags):
+    # cluster-sized diagonal blocks with a product for the rest of B between them
+    _solve(gpu, rng, n, nrhs, side | flags, pad=n & 1, alpha=0.75)
