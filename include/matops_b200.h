@@ -449,8 +449,8 @@ typedef struct mo_batch mo_batch;
 /* A plan for `count` square matrices of orders n[0..count) (host array, 1..MO_BATCH_MAX_N,
  * else MO_EBATCHN), each with nrhs right-hand sides (0: factor only).  The plan orders the
  * matrices longest first, groups them by the kernel configuration chosen for their size
- * bucket and records one CUDA graph (queue reset + one persistent kernel per group, the
- * group with the largest matrices first) on its first run. */
+ * bucket and records one CUDA graph (queue reset, then one persistent kernel per group, the
+ * groups side by side) on its first run. */
 MO_API int mo_batch_create(mo_ctx *ctx, int kind, int count, const int32_t *n, int nrhs,
                            mo_batch **plan);
 MO_API int mo_batch_destroy(mo_batch *plan);
@@ -464,8 +464,8 @@ MO_API int mo_batch_destroy(mo_batch *plan);
  * arrays updates the graph's kernel parameters instead of re-recording it. */
 MO_API int mo_batch_run(mo_batch *plan, double *const *A, const int64_t *lda, double *const *B,
                         const int64_t *ldb, int64_t *const *piv, int *info);
-/* Autotuner: for each size bucket in the plan, times every kernel configuration (panel
- * width 32 or 16, CTAs per SM) on synthetic matrices of the plan's own orders (`reps`
+/* Autotuner: for each size bucket in the plan, times every kernel configuration (0 or 1:
+ * more threads per matrix, or more matrices per SM) on synthetic matrices of the plan's own orders (`reps`
  * timed runs each, best kept) and keeps the fastest.  ms (optional, MO_BATCH_BUCKETS x 2
  * doubles) receives the times (-1 where a bucket is empty).  Synchronous. */
 MO_API int mo_batch_tune(mo_batch *plan, int reps, double *ms);
