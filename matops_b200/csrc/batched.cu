@@ -33,7 +33,7 @@
 // few warps can do is kept short.  Measured on B200, 4096 systems n ~ U{16..512}, 1 RHS,
 // against right-looking 32-column panels with shared-memory staging (diagonal block, panel
 // substitution and solve by division chains; LU panels unrolled over 32 columns):
-// Cholesky 9.8 -> 5.5 ms, LU 40.3 -> 16.4; 512 x n = 256 Cholesky 0.94 -> 0.45 ms, LU 3.86 -> 1.46;
+// Cholesky 9.8 -> 5.75 ms, LU 40.3 -> 16.3; 512 x n = 256 Cholesky 0.94 -> 0.45 ms, LU 3.86 -> 1.46;
 // 1024 x n = 128 Cholesky 0.67 -> 0.22, LU 2.51 -> 0.64.
 #include <algorithm>
 #include <cmath>

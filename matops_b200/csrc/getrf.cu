@@ -307,6 +307,7 @@ __device__ __forceinline__ void cl_argmax(unsigned &hi, unsigned &lo, int &idx) 
 // BY_WARP (at most kClByWarp CTAs): every warp sends its own candidate to every CTA, which spares
 // the second argmax level and a block barrier per column; more CTAs would receive more
 // candidates than a warp has lanes, and many times the bytes, so there a CTA sends one.
+// Panels of LU at n = 1001: 221 -> 214 us each.
 template <int RPT, bool BY_WARP>
 __global__ void __launch_bounds__(kClThreads, 1)
     lu_cluster_panel_kernel(double *P, int64_t ld, int m, int W, int64_t *piv, int64_t row0,

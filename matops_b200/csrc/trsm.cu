@@ -71,7 +71,7 @@ int trsm_sweeps(mo_ctx *ctx, View B, View A, int flags, double alpha, bool pair)
   const size_t flag_ints = (size_t)4 * 32 * ((N + 63) / 64) + 64;
   int rc = workspace(ctx, inv_bytes + sizeof(int) * flag_ints, (void **)&inv);
   if (rc) return rc;
-  // few right-hand sides: one cooperative launch instead of a sweep of 2*nblk GEMMs
+  // few right-hand sides: a few launches instead of a sweep of 2*nblk GEMMs
   if (nblk > 1 && nrhs <= 64)
     return trsm_few(ctx, B, A, flags, alpha, inv,
                     reinterpret_cast<int *>(reinterpret_cast<char *>(inv) + inv_bytes), pair);

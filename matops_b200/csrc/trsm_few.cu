@@ -1,4 +1,6 @@
-// Triangular solve with few right-hand sides (<= 64) in one cooperative launch.
+// Triangular solve with few right-hand sides (<= 64).  Orders and factors that fit go to
+// cluster-sized blocks (trsm_cluster.cuh; few_run and few_sweep hold the rules); this file's own
+// kernels do the others in one cooperative launch.
 //
 // op(A) X = alpha*B with op(A) n x n triangular, split into 64-row blocks.  The columns of
 // B are cut into groups of at most MO_FEW_GROUP (32), each solved by its own set of CTAs
