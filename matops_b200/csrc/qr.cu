@@ -257,7 +257,8 @@ struct ClQr {
   __align__(16) double sum[2][kClMaxCtas][32];
   __align__(16) double prow[2][32];
   __align__(16) double own[32], ownrow[32];  // gathered for sending
-  double red[kClWarps][32];
+  double red[2][kClWarps][32];     // each warp's sums, by column parity: one barrier per column
+                                   // does not keep a fast warp from writing the next column's
   __align__(16) double w[kClWarps][32];      // each warp's copy of the update row
   double z[32][33];                // dlarft vectors: z[j][c] = -tau_j v_c^T v_j, c < j
   double tau[32];
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
       }
     }
-    s.red[warp][lane] = acc[0];
+    s.red[par][warp][lane] = acc[0];
     if (nctas > 1 && tid == 0)
       mbar_arrive_expect_tx(&s.bar[par], (uint32_t)((nctas + 1) * 32 * sizeof(double)));
     // the pivot row (one of CTA 0's first 32) goes out beside the sums
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     if (nctas > 1) {
       if (warp == 1) {
 #pragma unroll
-        for (int g = 0; g < kClWarps; ++g) qv += s.red[g][lane];
+        for (int g = 0; g < kClWarps; ++g) qv += s.red[par][g][lane];
         s.own[lane] = qv;
         __syncwarp();
         cl_send<16>(s.sum[par][cta], s.own, &s.bar[par], lane, nctas);
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
       for (int g = 0; g < kClMaxCtas; ++g) qv += part[g];
     } else {
 #pragma unroll
-      for (int g = 0; g < kClWarps; ++g) qv += s.red[g][lane];
+      for (int g = 0; g < kClWarps; ++g) qv += s.red[par][g][lane];
     }
     const double prc = s.prow[par][lane];
     // computeHouseholder (house.go:55-78) on [alpha; x] with ||x||^2 = q_0, in every lane
