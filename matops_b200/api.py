@@ -518,18 +518,22 @@ class BatchPlan:
         if len(As) != count:
             raise ValueError("number of matrices does not match the plan")
         given = (bool(Bs), bool(pivs))
+        # a refused call leaves the host's table half filled: no device table then, so that the
+        # next one sends it whole
+        table, self._table = self._table, None
         changed = _lib.ext().batch_pack(As, Bs if given[0] else None, pivs if given[1] else None,
                                       self.orders.ctypes.data, count, self.nrhs,
                                       self._host.ctypes.data)
-        if changed or self._given != given or self._table is None:
+        if changed or self._given != given or table is None:
             dev = As[0].device if count else torch.device("cuda", torch.cuda.current_device())
-            self._table = None
+            table = None
             staged = torch.empty(5 * count, dtype=torch.int64, pin_memory=count > 0)
             staged.numpy()[:] = self._host
-            self._table = staged.to(dev, non_blocking=True)
+            table = staged.to(dev, non_blocking=True)
             self._info = torch.zeros(count, dtype=torch.int32, device=dev)
             self._given = given
             self._stream = torch.cuda.current_stream(dev).cuda_stream
+        self._table = table
         here = torch.cuda.current_stream(self._table.device)
         if here.cuda_stream != self._stream:  # not the stream the memory belongs to
             self._table.record_stream(here)
