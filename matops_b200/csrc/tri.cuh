@@ -141,11 +141,14 @@ __device__ __forceinline__ void tri_inv16(double *Xd, int ldc, int ldi, double r
       s1 = fma(-l(i, m + 1), x[m + 1], s1);
     }
     if (i & 1) s0 = fma(-l(i, i - 1), x[i - 1], s0);
-    x[i] = (s0 + s1) * __shfl_sync(0xffffffffu, rd, i);
+    const double r = __shfl_sync(0xffffffffu, rd, i);
+    // zero above the diagonal also where the row has a zero pivot (0 times infinity): the
+    // columns right of it are those of a regular triangle
+    x[i] = i < c ? 0.0 : (s0 + s1) * r;
   }
   if (lane < 16) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) Xd[c * ldc + i * ldi] = i < c ? 0.0 : x[i];
+    for (int i = 0; i < 16; ++i) Xd[c * ldc + i * ldi] = x[i];
   }
 }
 
