@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       const int r = rbase + kClThreads * q;
-      if (r > j) {  // (rows past R hold zeros)
+      if (r > j && r < R) {  // (rows past R hold zeros only while no NaN is about)
 #pragma unroll
         for (int k = 0; k < 32; ++k) acc[k] = fma(x[q][0], x[q][k], acc[k]);
       }
@@ -447,16 +447,39 @@ __global__ void __launch_bounds__(256) qr_t_block_kernel(double *Tb, int64_t ldt
   double *T = sm;                  // [128][kTbLd], zeros outside bo x bo and below the diagonal
   double *M1 = sm + 128 * kTbLd;   // [96][36]
   const int tid = threadIdx.x, warp = tid >> 5;
+  bool odd = false;
 #pragma unroll 16
   for (int e = tid; e < 128 * 128; e += 256) {
     const int r = e & 127, c = e >> 7;
     const bool own = r < bo && c < bo && r <= c && r / kQrPanel == c / kQrPanel;
     // above the diagonal panels: the Gram matrix, replaced block column by block column
     const bool gram = r < bo && c < bo && r / kQrPanel < c / kQrPanel;
-    T[r * kTbLd + c] = own ? Tb[r + (int64_t)c * ldt] : gram ? Zin[r + (int64_t)c * ldz] : 0.0;
+    const double v = own ? Tb[r + (int64_t)c * ldt] : gram ? Zin[r + (int64_t)c * ldz] : 0.0;
+    T[r * kTbLd + c] = v;
+    odd |= !isfinite(v);
   }
-  __syncthreads();
-  for (int p0 = kQrPanel; p0 < bo; p0 += kQrPanel) {
+  // with an infinity or a NaN about, the zeros below T's diagonal must not meet it: sums over
+  // T's upper triangle only, element by element, so that the columns left of it stay right
+  odd = __syncthreads_or(odd);
+  for (int p0 = kQrPanel; odd && p0 < bo; p0 += kQrPanel) {
+    const int w = min(kQrPanel, bo - p0);
+    for (int e = tid; e < p0 * w; e += 256) {
+      const int c = e / p0, r = e - c * p0;
+      double acc = 0.0;
+      for (int l = 0; l <= c; ++l)
+        acc = fma(T[r * kTbLd + p0 + l], T[(p0 + l) * kTbLd + p0 + c], acc);
+      M1[r * 36 + c] = acc;
+    }
+    __syncthreads();
+    for (int e = tid; e < p0 * w; e += 256) {
+      const int c = e / p0, r = e - c * p0;
+      double acc = 0.0;
+      for (int l = r; l < p0; ++l) acc = fma(T[r * kTbLd + l], M1[l * 36 + c], acc);
+      T[r * kTbLd + p0 + c] = -acc;
+    }
+    __syncthreads();
+  }
+  for (int p0 = kQrPanel; !odd && p0 < bo; p0 += kQrPanel) {
     const int nt = p0 / 16;  // 16-row tiles above the panel, two columns of them
     // M1 = Zin(0:p0, p0:p0+32) T(p0:p0+32, p0:p0+32)
     for (int t = warp; t < 2 * nt; t += 8) {
