@@ -408,6 +408,22 @@ __device__ __forceinline__ void lu_compact(LuSmem &s, int n, int lo) {
   }
 }
 
+// The unit lower 32 x 32 triangle at (jo, jo) on the rows of ut, 32 columns from c0, by forward
+// substitution, a lane per column, the result also to A (one warp): for right-hand sides with
+// an infinity or a NaN, which the zeros of an inverse would carry into the rows above
+__device__ __noinline__ void lu_substitute(const int *perm, double *A, int64_t ld, int n, int jo,
+                                           double *ut, int c0) {
+  const int c = c0 + (threadIdx.x & 31);
+  for (int i = 0; i < CB; ++i) {
+    double v = ut[(int64_t)i * UTLD + c];
+    const double *l = A + perm[jo + i] + (int64_t)jo * ld;
+    for (int k = 0; k < i; ++k) v = fma(-l[(int64_t)k * ld], ut[(int64_t)k * UTLD + c], v);
+    ut[(int64_t)i * UTLD + c] = v;
+    if (c < n) A[perm[jo + i] + (int64_t)c * ld] = v;
+  }
+  __syncwarp();
+}
+
 // U12 = L11^-1 A12 for the 64-row block at jo, by 32 rows: U_0 = inv(L_00) A_0, U_1 = inv(L_11)
 // (A_1 - L_10 U_0), a warp per 32 columns; written to the rows' physical places and row-major
 // into ut
@@ -465,11 +481,26 @@ __device__ __noinline__ void lu_u12(LuSmem &s, double *A, int64_t ld, int n, int
       return [=](int k, int ni) { return ut[(int64_t)(h + k) * UTLD + c0 + 8 * ni + g]; };
     };
     double acc[2][4][4];
+    int top = 0;  // largest exponent among the right-hand sides in hand
+    auto seen = [&](double v) {
+      top = max(top, __double2hiint(v) & 0x7fffffff);
+      return v;
+    };
+    auto odd = [&] { return __any_sync(0xffffffffu, top >= 0x7ff00000); };
     zero(acc);
     product(acc, &s.L[0][0], LB + 2, [&](int k, int ni) {
-      return A[s.perm[jo + k] + (int64_t)min(c0 + 8 * ni + g, n - 1) * ld];
+      return seen(A[s.perm[jo + k] + (int64_t)min(c0 + 8 * ni + g, n - 1) * ld]);
     });
-    store(acc, 0, 1.0, true);
+    if (odd()) {
+      const int c = min(c0 + lane, n - 1);
+      for (int i = 0; i < CB; ++i)
+        ut[(int64_t)i * UTLD + c0 + lane] = A[s.perm[jo + i] + (int64_t)c * ld];
+      __syncwarp();
+      lu_substitute(s.perm, A, ld, n, jo, ut, c0);
+      top = 0;
+    } else {
+      store(acc, 0, 1.0, true);
+    }
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
@@ -479,7 +510,17 @@ __device__ __noinline__ void lu_u12(LuSmem &s, double *A, int64_t ld, int n, int
           acc[mi][ni][q] = neg(A[s.perm[jo + CB + 16 * mi + g + 8 * (q >> 1)] +
                                  (int64_t)min(c0 + 8 * ni + 2 * t4 + (q & 1), n - 1) * ld]);
     product(acc, &s.L[0][CB], LB + 2, from_ut(0));
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) seen(acc[mi][ni][q]);
     store(acc, CB, -1.0, false);
+    if (odd()) {
+      lu_substitute(s.perm, A, ld, n, jo + CB, ut + (int64_t)CB * UTLD, c0);
+      continue;
+    }
     zero(acc);
     product(acc, &s.L[CB][CB], LB + 2, from_ut(CB));
     __syncwarp();  // every lane has read ut's rows before they are replaced
