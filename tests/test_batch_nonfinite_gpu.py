@@ -40,3 +40,15 @@ def test_batched_lu_spoilt_row_at_the_end_of_a_block(gpu, rng):
     gpu.BatchPlan(gpu.BATCH_LU, [n]).run(a, None, piv)
     out = a[0].cpu().numpy()
     assert np.isfinite(out[:63]).all() and not np.isfinite(out[63, 64])
+
+
+@pytest.mark.parametrize("n", [16, 32, 48, 64, 128])
+def test_batched_cholesky_zero_last_pivot(gpu, n):
+    # semidefinite, the zero in the last column: the root of zero is zero, as in the reference
+    # (only a pivot whose root is NaN is refused, chol.go:33-36)
+    A = np.diag(np.arange(1.0, n + 1))
+    A[n - 1, n - 1] = 0.0
+    a = [gpu.to_device(A)]
+    assert gpu.BatchPlan(gpu.BATCH_CHOL, [n]).run(a).tolist() == [0]
+    out = a[0].cpu().numpy()
+    assert fro(out - np.sqrt(A)) <= n * EPS * fro(A) and out[n - 1, n - 1] == 0.0
