@@ -89,11 +89,16 @@ def _call(form, name, *args):
     if entry is None:
         lib = _lib.lib()
         entry = _entry[name] = (getattr(_lib.ext(), form), _lib.address(getattr(lib, name)))
+    return entry[0](entry[1], *_current(), *args)
+
+
+def _current():
+    """address of the current device's context, and its current stream"""
     dev = torch.cuda.current_device()
     ctx = _handles.get(dev)
     if ctx is None:
         ctx = _handles[dev] = context(dev).value
-    return entry[0](entry[1], ctx, torch._C._cuda_getCurrentRawStream(dev), *args)
+    return ctx, torch._C._cuda_getCurrentRawStream(dev)
 
 
 def view(t: torch.Tensor) -> _lib.MoMatrix:
@@ -496,6 +501,9 @@ class BatchPlan:
             raise MatopsError(rc, _lib.lib().mo_strerror(rc).decode())
         self._host = np.zeros(5 * len(self.orders), dtype=np.int64)  # the table (see run)
         self._table = self._info = self._given = None
+        # (numpy makes an object for every look at an address, 0.7 us)
+        self._kept = self.orders
+        self._addr = self._kept.ctypes.data, self._host.ctypes.data
 
     def close(self):
         if self._h:
@@ -522,8 +530,7 @@ class BatchPlan:
         # next one sends it whole
         table, self._table = self._table, None
         changed = _lib.ext().batch_pack(As, Bs if given[0] else None, pivs if given[1] else None,
-                                      self.orders.ctypes.data, count, self.nrhs,
-                                      self._host.ctypes.data)
+                                      self._addr[0], count, self.nrhs, self._addr[1])
         if changed or self._given != given or table is None:
             dev = As[0].device if count else torch.device("cuda", torch.cuda.current_device())
             table = None
@@ -534,17 +541,17 @@ class BatchPlan:
             self._given = given
             self._stream = torch.cuda.current_stream(dev).cuda_stream
         self._table = table
-        here = torch.cuda.current_stream(self._table.device)
-        if here.cuda_stream != self._stream:  # not the stream the memory belongs to
-            self._table.record_stream(here)
+        # (raw stream handles: a stream object and context() cost 2 us each, a launch 8)
+        if torch._C._cuda_getCurrentRawStream(table.get_device()) != self._stream:
+            here = torch.cuda.current_stream(table.device)  # not the one the memory belongs to
+            table.record_stream(here)
             self._info.record_stream(here)
-        base = self._table.data_ptr()
-
-        def p(k, on=True):
-            return ctypes.c_void_p(base + 8 * k * count) if on else None
-        context()
-        rc = _lib.lib().mo_batch_run(self._h, p(0), p(1), p(2, given[0]), p(3, given[0]),
-                                     p(4, given[1]), ctypes.c_void_p(self._info.data_ptr()))
+        base, step = table.data_ptr(), 8 * count
+        lib = _lib.lib()
+        lib.mo_set_stream(*_current())
+        rc = lib.mo_batch_run(self._h, base, base + step, base + 2 * step if given[0] else None,
+                              base + 3 * step if given[0] else None,
+                              base + 4 * step if given[1] else None, self._info.data_ptr())
         if rc:
             raise MatopsError(rc, _lib.lib().mo_strerror(rc).decode())
         return self._info
