@@ -49,7 +49,7 @@ def build(verbose: bool = False, jobs: int = 8) -> str:
     """Compile every csrc/*.cu to an object (in parallel) and link the shared library."""
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(
+    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(
         os.path.join(HERE, "..", "include", "*.h"))
     procs, objs = [], []
     if _stale(EXT, [os.path.join(CSRC, "tensors.cpp")] + headers):

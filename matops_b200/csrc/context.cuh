@@ -21,6 +21,7 @@ struct mo_ctx {
   void *ws = nullptr;
   size_t ws_bytes = 0;
   int sms = 148;
+  int lu_ctas = 0;  // CTAs of the largest LU panel cluster the device places (0: not asked yet)
   // second, high-priority stream for look-ahead panels, and fork/join events
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -20,6 +20,7 @@
 
 #include "cluster.cuh"
 #include "context.cuh"
+#include "lu_shape.h"
 #include "tri.cuh"
 
 namespace mo {
@@ -266,8 +267,7 @@ __global__ void __launch_bounds__(PANEL_THREADS)
 // 320, 16000 rows 766 -> 439 (there the FP64 rate of the 16 SMs takes over).  A column takes
 // about 1000 cycles in one CTA and 1700 in a cluster, half of it the two argmax levels and
 // the exchange; the triangle of U and the left-looking products take the other third.
-constexpr int kClThreads = 256, kClWarps = kClThreads / 32, kClSub = 16, kClMaxCtas = 16;
-constexpr int kClMaxRows = kClThreads * kClMaxCtas * 4;
+constexpr int kClWarps = kClThreads / 32, kClSub = 16;
 constexpr int kClByWarp = 4, kClCands = kClByWarp * kClWarps;  // (one lane per candidate)
 constexpr int kClL = MAX_PANEL_W - kClSub;  // rows of U that a later sub-panel needs
 constexpr int kClLd = kClL + 2;  // a row of L^T (16-byte aligned, 4 banks from the next)
@@ -599,20 +599,6 @@ __global__ void __launch_bounds__(kClThreads, 1)
     mv_dst[at] = (int)row0 + r;
     mv_src[at] = (int)row0 + phys[q];
   }
-}
-
-// CTAs and rows per thread of the cluster panel for m <= kClMaxRows rows: one row per thread
-// while 16 CTAs suffice (a second and a fourth row per thread cost 50 and 130 us a panel at
-// 1001 rows, more CTAs 1 to 10 us; the step from one CTA to a cluster costs 65 us, a row
-// more per thread the same)
-inline int cl_shape(int m, int *rpt) {
-  int c = 1, r = 1;
-  while (c * kClThreads * r < m) {
-    if (c < kClMaxCtas) c *= 2;
-    else r *= 2;
-  }
-  *rpt = r;
-  return c;
 }
 
 const void *cl_kernel(int ctas, int rpt) {
@@ -968,25 +954,33 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
     q += 2 * (2 * MAX_PANEL_W) * sizeof(int) + 64;
   }
 
-  // rows up to which a panel may run in one cluster (the 16-CTA cluster is not portable: ask)
-  int cl_rows = kClThreads * 8 * 4;
-  if (m > cl_rows) {
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    int clusters = 0;
-    if ((rc = cl_config(kClMaxCtas, 4, ctx->stream, &cfg, &attr))) return rc;
-    if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(kClMaxCtas, 4), &cfg) == cudaSuccess &&
-        clusters > 0)
-      cl_rows = kClMaxRows;
-    else
-      cudaGetLastError();
+  // CTAs and rows up to which a panel may run in one cluster.  More than 8 CTAs are not portable
+  // (a part of a device may not place them): ask, once per context, where they would be used.
+  int cl_ctas = kClPortable;
+  if (m > kClThreads * kClPortable) {
+    if (ctx->lu_ctas == 0) {
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr;
+      int clusters = 0;
+      if ((rc = cl_config(kClMaxCtas, kClMaxRpt, ctx->stream, &cfg, &attr))) return rc;
+      if (cudaOccupancyMaxActiveClusters(&clusters, cl_kernel(kClMaxCtas, kClMaxRpt), &cfg) ==
+              cudaSuccess &&
+          clusters > 0) {
+        ctx->lu_ctas = kClMaxCtas;
+      } else {
+        cudaGetLastError();
+        ctx->lu_ctas = kClPortable;
+      }
+    }
+    cl_ctas = ctx->lu_ctas;
   }
+  const int cl_rows = cl_max_rows(cl_ctas);
   // one panel: factor A[k:m, k:k+b] and list its interchanges
   auto panel = [&](int k, int b, Moves &v) -> int {
     v.own = m - k <= cl_rows;
     if (v.own) {
       int rpt;
-      const int ctas = cl_shape(m - k, &rpt);
+      const int ctas = cl_shape(m - k, cl_ctas, &rpt);
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute attr;
       int r2 = cl_config(ctas, rpt, ctx->stream, &cfg, &attr);
