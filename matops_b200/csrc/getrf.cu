@@ -1012,6 +1012,7 @@ int getrf(mo_ctx *ctx, View A, int64_t *piv, int64_t npiv, int ref_nb) {
     MO_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)lu_panel_kernel, dim3(pblk),
                                             dim3(PANEL_THREADS), args, smem, ctx->stream));
     prof_end(ctx, ps, (double)pm * b * b - (double)b * b * b / 3.0, 16.0 * pm * b);
+    if (n <= b) return MO_OK;  // no other columns to interchange rows in
     ProfScope pms;
     prof_begin(ctx, pms, MO_PROF_LASWP);
     if (m - k <= kSwapTableMax) {
