@@ -411,6 +411,193 @@ __global__ void __launch_bounds__(ABT, 4) adj_batch_kernel(AdjBatchArgs p) {
   }
 }
 
+// The same sweep with all warps of a CTA of 256 threads in step on every product (FP64 FMA over
+// tiles staged in shared memory, 4 outputs per thread): its chain per 32 columns is half as
+// long as one warp's DMMA products and inverses, and its rate lower.  For few or small
+// matrices, where the chain is the time.  The rule is adj_by_fma's.
+constexpr int kAdjFmaThreads = 256, kAdjFmaLd = AB + 1;
+
+struct AdjFmaSmem {
+  double As[AB][kAdjFmaLd], Bs[AB][kAdjFmaLd];    // GEMM staging
+  double Dm[AB][kAdjFmaLd], Di[AB][kAdjFmaLd];    // D (lower, identity padded) and D^-1
+  double X1[AB][kAdjFmaLd], X2[AB][kAdjFmaLd];    // the adjoint of chol(D)
+  int idx;
+};
+
+// C (M x N, ldc) += alpha op(A) op(B), op(A) M x K, op(B) K x N; `lower`: only i >= j.
+// op(A)(i, k) = ta ? A[k + i lda] : A[i + k lda]; op(B)(k, j) = tb ? B[j + k ldb] : B[k + j ldb].
+// C must not overlap A or B.  Ends with a barrier.
+__device__ void adj_fma_gemm(AdjFmaSmem &s, int M, int N, int K, double alpha, const double *A,
+                             int64_t lda, bool ta, const double *B, int64_t ldb, bool tb, double *C,
+                             int64_t ldc, bool lower) {
+  const int tid = threadIdx.x, r = tid & 31, cg = tid >> 5;  // row r, columns 4 cg .. + 3
+  for (int i0 = 0; i0 < M; i0 += AB)
+    for (int j0 = 0; j0 < N; j0 += AB) {
+      if (lower && j0 > i0 + AB - 1) continue;
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k0 = 0; k0 < K; k0 += AB) {
+        __syncthreads();
+        for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+          const int a = e & 31, b = e >> 5;
+          const int ii = ta ? b : a, ka = ta ? a : b;  // consecutive threads: consecutive addresses
+          const int gi = i0 + ii, gk = k0 + ka;
+          s.As[ii][ka] = (gi < M && gk < K) ? (ta ? A[gk + (int64_t)gi * lda] : A[gi + (int64_t)gk * lda]) : 0.0;
+          const int kb = tb ? b : a, jj = tb ? a : b;
+          const int gk2 = k0 + kb, gj = j0 + jj;
+          s.Bs[kb][jj] = (gk2 < K && gj < N) ? (tb ? B[gj + (int64_t)gk2 * ldb] : B[gk2 + (int64_t)gj * ldb]) : 0.0;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < AB; ++k) {
+          const double av = s.As[r][k];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[c] = fma(av, s.Bs[k][4 * cg + c], acc[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int gi = i0 + r, gj = j0 + 4 * cg + c;
+        if (gi < M && gj < N && (!lower || gi >= gj)) C[gi + (int64_t)gj * ldc] += alpha * acc[c];
+      }
+    }
+  __syncthreads();
+}
+
+// Z = op(X) op(Y) for 32 x 32 shared-memory blocks (Z distinct from X and Y); ends with a barrier
+__device__ void adj_fma_mm32(double (*Z)[kAdjFmaLd], const double (*X)[kAdjFmaLd], bool tx,
+                             const double (*Y)[kAdjFmaLd], bool ty) {
+  const int tid = threadIdx.x, r = tid & 31, cg = tid >> 5;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 8
+  for (int k = 0; k < AB; ++k) {
+    const double xv = tx ? X[k][r] : X[r][k];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c] = fma(xv, ty ? Y[4 * cg + c][k] : Y[k][4 * cg + c], acc[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) Z[r][4 * cg + c] = acc[c];
+  __syncthreads();
+}
+
+// the reverse sweep of one matrix by the whole CTA
+__device__ void adj_fma_matrix(AdjFmaSmem &s, const double *L, int64_t ldl, double *G, int64_t ldg,
+                               int n) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int last = ((n - 1) / AB) * AB;
+  for (int j0 = last; j0 >= 0; j0 -= AB) {
+    const int jb = min(AB, n - j0), below = n - j0 - jb;
+    const double *D = L + j0 + (int64_t)j0 * ldl;
+    double *Dbar = G + j0 + (int64_t)j0 * ldg;
+    for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+      const int i = e & 31, j = e >> 5;
+      s.Dm[i][j] = (i < jb && j < jb) ? (i >= j ? D[i + (int64_t)j * ldl] : 0.0) : (i == j ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    // D^-1 (lower): lane c of warp 0 solves D x = e_c
+    if (warp == 0) {
+      const double rdi = 1.0 / s.Dm[lane][lane];
+      double x[AB];
+#pragma unroll
+      for (int i = 0; i < AB; ++i) {
+        double s0 = (i == lane) ? 1.0 : 0.0, s1 = 0.0;
+#pragma unroll
+        for (int m = 0; m + 1 < i; m += 2) {
+          s0 = fma(-s.Dm[i][m], x[m], s0);
+          s1 = fma(-s.Dm[i][m + 1], x[m + 1], s1);
+        }
+        if (i & 1) s0 = fma(-s.Dm[i][i - 1], x[i - 1], s0);
+        const double rd = __shfl_sync(0xffffffffu, rdi, i);
+        x[i] = (i < lane) ? 0.0 : (s0 + s1) * rd;
+      }
+#pragma unroll
+      for (int i = 0; i < AB; ++i) s.Di[i][lane] = x[i];
+    }
+    __syncthreads();
+    if (below > 0) {
+      double *Bbar = G + (j0 + jb) + (int64_t)j0 * ldg;
+      const double *B = L + (j0 + jb) + (int64_t)j0 * ldl;
+      // Bbar <- Bbar D^-1 in 32-row chunks through the staging tiles
+      for (int r0 = 0; r0 < below; r0 += AB) {
+        for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+          const int i = e & 31, k = e >> 5;
+          s.As[i][k] = (r0 + i < below && k < jb) ? Bbar[(r0 + i) + (int64_t)k * ldg] : 0.0;
+        }
+        __syncthreads();
+        adj_fma_mm32(s.Bs, s.As, false, s.Di, false);
+        for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+          const int i = e & 31, j = e >> 5;
+          if (r0 + i < below && j < jb) Bbar[(r0 + i) + (int64_t)j * ldg] = s.Bs[i][j];
+        }
+        __syncthreads();
+      }
+      adj_fma_gemm(s, jb, jb, below, -1.0, Bbar, ldg, true, B, ldl, false, Dbar, ldg, true);
+      if (j0 > 0) {
+        adj_fma_gemm(s, below, j0, jb, -1.0, Bbar, ldg, false, L + j0, ldl, false, G + (j0 + jb), ldg,
+                 false);  // Cbar -= Bbar R
+        adj_fma_gemm(s, jb, j0, below, -1.0, Bbar, ldg, true, L + (j0 + jb), ldl, false, G + j0, ldg,
+                 false);  // Rbar -= Bbar^T C
+      }
+    }
+    // adjoint of chol(D): S = D^-T Phi(D^T tril(Dbar)) D^-1
+    for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+      const int i = e & 31, j = e >> 5;
+      s.X1[i][j] = (i < jb && j < jb && i >= j) ? Dbar[i + (int64_t)j * ldg] : 0.0;
+    }
+    __syncthreads();
+    adj_fma_mm32(s.X2, s.Dm, true, s.X1, false);
+    for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+      const int i = e & 31, j = e >> 5;
+      s.X2[i][j] = i > j ? s.X2[i][j] : (i == j ? 0.5 * s.X2[i][j] : 0.0);
+    }
+    __syncthreads();
+    adj_fma_mm32(s.X1, s.X2, false, s.Di, false);
+    adj_fma_mm32(s.X2, s.Di, true, s.X1, false);
+    // E = S + S^T; Dbar (lower) = Phi-like copy of E
+    for (int e = tid; e < AB * AB; e += kAdjFmaThreads) {
+      const int i = e & 31, j = e >> 5;
+      const double v = s.X2[i][j] + s.X2[j][i];
+      s.X1[i][j] = v;
+      if (i < jb && j < jb && i >= j) Dbar[i + (int64_t)j * ldg] = i == j ? 0.5 * v : v;
+    }
+    __syncthreads();
+    if (j0 > 0)  // Rbar -= E R
+      adj_fma_gemm(s, jb, j0, jb, -1.0, &s.X1[0][0], kAdjFmaLd, true, L + j0, ldl, false, G + j0, ldg, false);
+  }
+  // lower-entry adjoint -> symmetric gradient
+  for (int64_t e = tid; e < (int64_t)n * n; e += kAdjFmaThreads) {
+    const int i = (int)(e % n), j = (int)(e / n);
+    if (i > j) {
+      const double v = 0.5 * G[i + (int64_t)j * ldg];
+      G[i + (int64_t)j * ldg] = v;
+      G[j + (int64_t)i * ldg] = v;
+    }
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kAdjFmaThreads) adj_fma_kernel(AdjBatchArgs p) {
+  extern __shared__ __align__(16) unsigned char adj_smem_raw[];
+  AdjFmaSmem &s = *reinterpret_cast<AdjFmaSmem *>(adj_smem_raw);
+  for (;;) {
+    if (threadIdx.x == 0) s.idx = atomicAdd(p.counter, 1);
+    __syncthreads();
+    const int q = s.idx;
+    __syncthreads();
+    if (q >= p.count) break;
+    const int m = p.order[q];
+    adj_fma_matrix(s, p.L[m], p.ldl[m], p.G[m], p.ldg[m], p.n[m]);
+  }
+}
+
+// Which of the two kernels a batch takes, by its largest order and its number of matrices.
+// Measured on B200, all of one order, FMA / DMMA in us: 32: 1 matrix 14 / 31, 148 17 / 34, 600
+// 40 / 58; 64: 29 / 61, 33 / 65, 94 / 127; 96: 53 / 100, 60 / 109, 216 / 291; 100: 84 / 125,
+// 93 / 132, and 300 206 / 158; 160: 164 / 219, 193 / 271, 437 / 328; 256: 566 / 619, 710 / 764,
+// 1500 / 945; 320: 1076 / 1100, 1351 / 1431, 2974 / 1823; 400: 2222 / 2023, 3351 / 3064, 6489 / 3526.
+bool adj_by_fma(int nmax, int count, int sms) {
+  return nmax <= 96 || (nmax <= 320 && count <= sms);
+}
+
 size_t scratch_doubles() { return 5 * (size_t)NBA * NBA; }
 
 AdjScratch carve(double *base) {
@@ -522,13 +709,17 @@ extern "C" int mo_decompose_chol_adjoint_batched(mo_ctx *ctx, int count, const m
     a.ldl = d64 + ns;
     a.G = reinterpret_cast<double *const *>(d64 + 2 * ns);
     a.ldg = d64 + 3 * ns;
-    if ((rc = mo_smem_attr((const void *)adj_batch_kernel, (int)sizeof(AdjSmem)))) return rc;
+    const bool fma = adj_by_fma(L[small[0]].rows, ns, ctx->sms);
+    const auto kernel = fma ? adj_fma_kernel : adj_batch_kernel;
+    const int threads = fma ? kAdjFmaThreads : ABT;
+    const size_t smem = fma ? sizeof(AdjFmaSmem) : sizeof(AdjSmem);
+    if ((rc = mo_smem_attr((const void *)kernel, (int)smem))) return rc;
     int occ = 0;
-    MO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, adj_batch_kernel, ABT, sizeof(AdjSmem)));
+    MO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
     const int grid = std::max(1, std::min(ns, ctx->sms * std::max(1, occ)));
     ProfScope ps;
     prof_begin(ctx, ps, MO_PROF_BATCH);
-    adj_batch_kernel<<<grid, ABT, sizeof(AdjSmem), main>>>(a);
+    kernel<<<grid, threads, smem, main>>>(a);
     double fl = 0.0;
     for (int i : small) fl += 2.0 * L[i].rows * (double)L[i].rows * L[i].rows / 3.0;
     prof_end(ctx, ps, fl, 0.0);
