@@ -779,20 +779,27 @@ size_t gemm_partial_bytes(int sms) { return 2 * (size_t)sms * TILE_DBL * sizeof(
 // Up to 2^27 multiply-adds the engine's start (barriers, tensor maps, the first slabs) and its
 // large tiles on a few SMs cost more than the small tiles' extra operand traffic.  Measured,
 // engine / small tiles in us: 64^3 12.3 / 4.1, 512 x 128 x 128 18.4 / 6.2, 1000 x 1000 x 128 24.6 /
-// 19.3, 500^3 32.8 / 18.4; above, 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  A C of a few
-// small tiles with a long K is split along K, two CTAs per SM with at least 128 rows of K each,
-// and the partial tiles are added in order by a second kernel, up to 2^29
-// multiply-adds: 128 x 128 x 8000 219 / 21, 512 x 128 x 8000 103 / 62, 1000 x 128 x 8000 101 / 119.
+// 19.3, 500^3 32.8 / 18.4; above, 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  With A
+// transposed and B not, both operands' loads run across their columns, and past 1500 tiles the
+// small ones lose where there is more than one slab: 1414 x 1414 x 16 10.9 / 10.4, x 30 14.4 /
+// 16.5, x 68 20.6 / 26.7; 1000 x 1000 x 30, 1024 tiles, 12.5 / 10.3.
+// A C of a few small tiles with a long K is split along K, two CTAs per SM with at least 128
+// rows of K each, and the partial tiles are added in order by a second kernel: up to 2^29
+// multiply-adds, 128 x 128 x 8000 219 / 21, 512 x 128 x 8000 103 / 62, 1000 x 128 x 8000 101 / 119;
+// up to 2^31 for at most 16 tiles, where the engine has one owner adding most SMs' partial
+// sums: 64 x 64 x 200000 575 / 96, 128 x 128 x 100000 335 / 171, 100 x 100 x 200000 439 / 341
+// (with odd leading dimensions 453 / 432), above it 128 x 128 x 200000 434 / 330 and 449 / 512.
 static int small_chunks(const GemmArgs &a, int sms) {
   const double tri = a.mode == kSyrkLower || a.mode == kSyrkUpper ? 0.5 : 1.0;
   const double work = tri * a.M * (double)a.N * a.K;
   if (a.force_fallback || a.N > 65535 * 32) return 0;
   const long long tiles = (long long)((a.M + 31) / 32) * ((a.N + 31) / 32);
   if (a.mode == kGemm && a.sk_partial && a.C != a.A && a.C != a.B && a.K >= 512 && tiles < sms &&
-      work <= 536870912.0) {
+      work <= (tiles <= 16 ? 2147483648.0 : 536870912.0)) {
     const int chunks = (int)std::min<long long>(a.K / 128, 2 * sms / tiles);
     if (chunks > 1) return chunks;
   }
+  if (a.transA && !a.transB && a.C != a.B && tri * tiles > 1500 && a.K > BK) return 0;
   return a.K <= 4096 && work <= 134217728.0 ? 1 : 0;
 }
 
