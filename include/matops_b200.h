@@ -99,12 +99,12 @@ MO_API int mo_num_workers(mo_ctx *ctx, int n);
  * 28-56 vs 96-121).  Returns the old value. */
 MO_API int mo_set_syrk_blas_beta(mo_ctx *ctx, int on);
 /* No counterpart in the reference (its calls cannot wait on another thread of work): the
- * number of polls a device-side wait on another CTA's step flag makes before it gives up
- * and records MO_EDEVTIMEOUT (the triangular solves with at most 64 right-hand sides, i.e.
- * SolveCHOL / SolveTrm with few columns and the refinement of mo_dsposv_ir).  Default
- * MO_SPIN_LIMIT_DEFAULT; a failing wait ends its kernel early, leaves no copy in flight and
- * the context stays usable (mo_sync returns MO_EDEVTIMEOUT once, the next call runs
- * normally).  *old (optional) receives the previous value. */
+ * number of polls a device-side wait on another CTA's step flag, or on its part of X, makes
+ * before it gives up and records MO_EDEVTIMEOUT (the triangular solves with at most 64
+ * right-hand sides, i.e. SolveCHOL / SolveTrm with few columns and the refinement of
+ * mo_dsposv_ir).  Default MO_SPIN_LIMIT_DEFAULT; a failing wait ends its kernel early, leaves no
+ * copy in flight and the context stays usable (mo_sync returns MO_EDEVTIMEOUT once, the next
+ * call runs normally).  *old (optional) receives the previous value. */
 #define MO_SPIN_LIMIT_DEFAULT (1u << 26)
 MO_API int mo_set_spin_limit(mo_ctx *ctx, uint32_t polls, uint32_t *old);
 

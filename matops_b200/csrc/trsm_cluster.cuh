@@ -23,29 +23,29 @@ constexpr int kTcThreads = 256, kTcBlock = 128, kTcMax = 16, kTcLd = kTcBlock + 
 template <int NR>
 struct TcSmem {
   uint64_t bar[kTcMax];                              // arrival of step s's x
+  int late;                                          // a wait of this CTA ran out
   __align__(16) double x[kTcMax][NR * kTcBlock];     // x of the earlier steps, by right-hand side
   __align__(16) double own[NR * kTcBlock];           // this CTA's x, and b before it
   double part[NR * kTcBlock];
   double inv[kTcBlock * kTcLd];                      // inv[k * kTcLd + i] = inverse(i, k)
 };
 
-// The wait for a step's x: with fewer polls than usual allowed (mo_set_spin_limit) one that runs
-// out is recorded, and the x still waited for, since it lands in this CTA's memory either way.
-__device__ __forceinline__ void tc_wait(uint64_t *bar, const FewArgs &p) {
-  if (p.spin_limit < MO_SPIN_LIMIT) {
-    for (uint32_t it = 0; it <= p.spin_limit; ++it) {
-      uint32_t done;
-      asm volatile(
-          "{\n\t.reg .pred q;\n\tmbarrier.test_wait.parity.shared::cta.b64 q, [%1], 0;\n\t"
-          "selp.u32 %0, 1, 0, q;\n\t}"
-          : "=r"(done)
-          : "r"(smem_u32(bar))
-          : "memory");
-      if (done) return;
-    }
-    set_status(p.status, MO_EDEVTIMEOUT);
+// The wait for step t's x (every thread waits for itself).  False, and the timeout recorded, when
+// the polls that the context allows (mo_set_spin_limit) run out.
+__device__ __forceinline__ bool tc_wait(uint64_t *bar, const FewArgs &p) {
+  if (p.spin_limit >= MO_SPIN_LIMIT) return mbar_wait(bar, 0, p.status);
+  for (uint32_t it = 0; it <= p.spin_limit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tmbarrier.test_wait.parity.shared::cta.b64 q, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bar))
+        : "memory");
+    if (done) return true;
   }
-  mbar_wait(bar, 0, p.status);
+  set_status(p.status, MO_EDEVTIMEOUT);
+  return false;
 }
 
 template <typename TA, bool TRANS, int NR>
@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
   };
   if (c > 0 && c < nblk) fetch(0);
   if (tid == 0) {
+    s.late = 0;
     for (int t = 0; t < kTcMax; ++t) mbar_init(&s.bar[t], 1);
     fence_barrier_init();
     for (int t = 0; t < c && c < nblk; ++t)
@@ -108,7 +109,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
   }
   if (c < nblk) {
     for (int t = 0; t < c; ++t) {
-      tc_wait(&s.bar[t], p);
+      if (!tc_wait(&s.bar[t], p)) {
+        s.late = 1;
+        break;
+      }
       if constexpr (!TRANS) {
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -164,43 +168,51 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
       }
     }
     __syncthreads();
-    if (h == 0) {
+    // A CTA that gave up leaves its rows as they are and sends NaN at once: the others' waits end,
+    // and its own memory is written until their x is here (waited for below).
+    const bool late = s.late;
+    if (late) {
+      for (int e = tid; e < NR * kTcBlock; e += kTcThreads)
+        s.own[e] = __longlong_as_double(0x7ff8000000000000ll);
+    } else {
+      if (h == 0) {
 #pragma unroll
-      for (int q = 0; q < NR; ++q) {
-        const double b = r < nrow && q < nr ? p.alpha * p.B[(int64_t)(r0 + r) * p.brs +
-                                                           (int64_t)(rhs0 + q) * p.bcs]
-                                            : 0.0;
-        s.own[q * kTcBlock + r] = b - (TRANS ? s.part[q * kTcBlock + r]
-                                             : acc[q] + s.part[q * kTcBlock + r]);
+        for (int q = 0; q < NR; ++q) {
+          const double b = r < nrow && q < nr ? p.alpha * p.B[(int64_t)(r0 + r) * p.brs +
+                                                             (int64_t)(rhs0 + q) * p.bcs]
+                                              : 0.0;
+          s.own[q * kTcBlock + r] = b - (TRANS ? s.part[q * kTcBlock + r]
+                                               : acc[q] + s.part[q * kTcBlock + r]);
+        }
       }
-    }
-    __syncthreads();
-    // x = inverse b
-    double x[NR];
+      __syncthreads();
+      // x = inverse b
+      double x[NR];
 #pragma unroll
-    for (int q = 0; q < NR; ++q) x[q] = 0.0;
-    const double *iv = s.inv + 64 * h * kTcLd + r;
-    // (the inverse's 64 x 64 block of zeros is left out: an infinity in b stays on its side)
-    if (h == (r >> 6) || (h == 0) == (p.lower_eff != 0)) {
+      for (int q = 0; q < NR; ++q) x[q] = 0.0;
+      const double *iv = s.inv + 64 * h * kTcLd + r;
+      // (the inverse's 64 x 64 block of zeros is left out: an infinity in b stays on its side)
+      if (h == (r >> 6) || (h == 0) == (p.lower_eff != 0)) {
 #pragma unroll 16
-      for (int k = 0; k < 64; ++k) {
-        const double v = iv[k * kTcLd];
+        for (int k = 0; k < 64; ++k) {
+          const double v = iv[k * kTcLd];
 #pragma unroll
-        for (int q = 0; q < NR; ++q) x[q] = fma(v, s.own[q * kTcBlock + 64 * h + k], x[q]);
+          for (int q = 0; q < NR; ++q) x[q] = fma(v, s.own[q * kTcBlock + 64 * h + k], x[q]);
+        }
       }
-    }
-    if (h == 1) {
+      if (h == 1) {
 #pragma unroll
-      for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
-    }
-    __syncthreads();
-    if (h == 0) {
+        for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
+      }
+      __syncthreads();
+      if (h == 0) {
 #pragma unroll
-      for (int q = 0; q < NR; ++q) {
-        const double v = r < nrow ? x[q] + s.part[q * kTcBlock + r] : 0.0;
-        s.own[q * kTcBlock + r] = v;
-        if (r < nrow && q < nr)
-          p.B[(int64_t)(r0 + r) * p.brs + (int64_t)(rhs0 + q) * p.bcs] = v;
+        for (int q = 0; q < NR; ++q) {
+          const double v = r < nrow ? x[q] + s.part[q * kTcBlock + r] : 0.0;
+          s.own[q * kTcBlock + r] = v;
+          if (r < nrow && q < nr)
+            p.B[(int64_t)(r0 + r) * p.brs + (int64_t)(rhs0 + q) * p.bcs] = v;
+        }
       }
     }
     __syncthreads();
@@ -218,6 +230,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
             : "memory");
       }
     }
+    if (late)
+      for (int t = 0; t < c; ++t) mbar_wait(&s.bar[t], 0, p.status);
   }
   cl_sync();  // no CTA leaves while another may still write into its memory
 }
