@@ -428,7 +428,8 @@ MO_API int mo_lp_gemm(mo_ctx *ctx, int prec, int64_t M, int64_t N, int64_t K, fl
  * Asynchronous on the context's stream. */
 MO_API int mo_decompose_chol_adjoint(mo_ctx *ctx, mo_matrix L, mo_matrix Lbar, int flags);
 /* The same for `count` independent matrices (host arrays of views), spread over a pool of
- * streams forked from and joined back into the context's stream. */
+ * streams forked from and joined back into the context's stream.  MO_ECUDA while that stream is
+ * being captured: the views' table is uploaded from host memory of the call. */
 MO_API int mo_decompose_chol_adjoint_batched(mo_ctx *ctx, int count, const mo_matrix *L,
                                              const mo_matrix *Lbar, int flags);
 /* Adjoint of X = A^-1 B solved with the factor L (SolveCHOL LOWER): Xbar (n x nrhs) is

@@ -582,7 +582,8 @@ def DecomposeCHOLAdjoint(L, Lbar, flags: int = LOWER):
 
 
 def DecomposeCHOLAdjointBatched(Ls, Lbars, flags: int = LOWER):
-    """DecomposeCHOLAdjoint for lists of independent matrices (one call, a pool of streams)."""
+    """DecomposeCHOLAdjoint for lists of independent matrices (one call, a pool of streams).
+    Not while a stream is being captured: the table of matrices goes up from host memory."""
     n, Lbars = len(Ls), list(Lbars)
     if len(Lbars) > max(n, 1):
         raise IndexError("more adjoints than factors")

@@ -650,6 +650,10 @@ extern "C" int mo_decompose_chol_adjoint_batched(mo_ctx *ctx, int count, const m
     if (G[i].rows != L[i].rows) return MO_ESIZE;
   }
   if (count == 0) return MO_OK;
+  // the table of views is uploaded from this call's memory: a graph would read it after its end
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  MO_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return MO_ECUDA;
   // orders up to kAdjBatchMaxN: one persistent kernel over a longest-first queue; larger
   // ones: the single-matrix sweep, spread over a pool of streams
   std::vector<int> small, big;
