@@ -13,6 +13,8 @@
 // right-hand side 15 us (36 us); n = 1001, three 45 us (93 us).  SolveTrm as a whole, block
 // inverses (24 us) included: n = 2048, one right-hand side 170 -> 55 us, 16: 168 -> 89 us.
 #pragma once
+#include <type_traits>
+
 #include "cluster.cuh"
 
 namespace mo {
@@ -48,7 +50,7 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, const FewArgs &p) {
   return false;
 }
 
-template <typename TA, bool TRANS, int NR>
+template <typename TA, bool TRANS, int NR, bool UNIT>
 __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewArgs p) {
   extern __shared__ __align__(16) unsigned char tc_raw[];
   TcSmem<NR> &s = *reinterpret_cast<TcSmem<NR> *>(tc_raw);
@@ -96,6 +98,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
       const double v = u < nrow && w < nrow ? iv[e] : 0.0;
       if (p.inv_t) s.inv[u * kTcLd + w] = v;
       else s.inv[w * kTcLd + u] = v;
+    }
+    if constexpr (UNIT) {
+      // op(A) itself between the two 64 x 64 diagonal blocks (see below)
+      __syncthreads();
+      const int i0 = p.lower_eff ? 64 : 0, k0 = 64 - i0;
+#pragma unroll 8
+      for (int e = tid; e < 64 * 64; e += kTcThreads) {
+        const int i = i0 + (TRANS ? e >> 6 : e & 63), k = k0 + (TRANS ? e & 63 : e >> 6);
+        const int64_t at = TRANS ? r0 + k + (int64_t)(r0 + i) * p.lda
+                                 : r0 + i + (int64_t)(r0 + k) * p.lda;
+        s.inv[k * kTcLd + i] = i < nrow && k < nrow ? (double)A[at] : 0.0;
+      }
     }
   }
   cl_sync();  // every CTA's barriers are armed before any x is sent
@@ -168,28 +182,65 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
       }
     }
     __syncthreads();
-    // A CTA that gave up leaves its rows as they are and sends NaN at once: the others' waits end,
-    // and its own memory is written until their x is here (waited for below).
-    const bool late = s.late;
-    if (late) {
-      for (int e = tid; e < NR * kTcBlock; e += kTcThreads)
-        s.own[e] = __longlong_as_double(0x7ff8000000000000ll);
-    } else {
-      if (h == 0) {
+    if (h == 0) {
 #pragma unroll
-        for (int q = 0; q < NR; ++q) {
-          const double b = r < nrow && q < nr ? p.alpha * p.B[(int64_t)(r0 + r) * p.brs +
-                                                             (int64_t)(rhs0 + q) * p.bcs]
-                                              : 0.0;
-          s.own[q * kTcBlock + r] = b - (TRANS ? s.part[q * kTcBlock + r]
-                                               : acc[q] + s.part[q * kTcBlock + r]);
-        }
+      for (int q = 0; q < NR; ++q) {
+        const double b = r < nrow && q < nr ? p.alpha * p.B[(int64_t)(r0 + r) * p.brs +
+                                                           (int64_t)(rhs0 + q) * p.bcs]
+                                            : 0.0;
+        s.own[q * kTcBlock + r] = b - (TRANS ? s.part[q * kTcBlock + r]
+                                             : acc[q] + s.part[q * kTcBlock + r]);
       }
-      __syncthreads();
-      // x = inverse b
-      double x[NR];
+    }
+    __syncthreads();
+    // x = inverse b, or for a unit diagonal by 64 rows: the inverse of a unit triangle grows
+    // with its order, and with it the error (n = 1001, L of a partially pivoted LU, against 64
+    // bits: 9.2e-15 by 128 rows, 6.6e-15 by 64; other factors by 128 rows are the closer ones)
+    double x[NR];
 #pragma unroll
-      for (int q = 0; q < NR; ++q) x[q] = 0.0;
+    for (int q = 0; q < NR; ++q) x[q] = 0.0;
+    if constexpr (UNIT) {
+      const int first = p.lower_eff ? 0 : 1;
+      // rows 64 ra .. times columns 64 ca .. of s.inv and s.own, 32 columns by each h; for h = 0
+      // in x
+      auto product = [&](int ra, int ca) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) x[q] = 0.0;
+        const int k0 = 64 * ca + 32 * h;
+        if ((r >> 6) == ra) {
+#pragma unroll 8
+          for (int k = k0; k < k0 + 32; ++k) {
+            const double v = s.inv[k * kTcLd + r];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) x[q] = fma(v, s.own[q * kTcBlock + k], x[q]);
+          }
+          if (h == 1) {
+#pragma unroll
+            for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
+          }
+        }
+        __syncthreads();
+        if ((r >> 6) == ra && h == 0) {
+#pragma unroll
+          for (int q = 0; q < NR; ++q) x[q] += s.part[q * kTcBlock + r];
+        }
+      };
+      for (int step = 0; step < 3; ++step) {
+        const int ra = step == 0 ? first : 1 - first, ca = step == 2 ? 1 - first : first;
+        product(ra, ca);
+        if ((r >> 6) == ra && h == 0) {
+#pragma unroll
+          for (int q = 0; q < NR; ++q) {
+            double &to = s.own[q * kTcBlock + r];
+            to = step == 1 ? to - x[q] : x[q];
+          }
+        }
+        __syncthreads();
+      }
+      // (as the sum of the two halves below)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) x[q] = h == 0 ? s.own[q * kTcBlock + r] : 0.0;
+    } else {
       const double *iv = s.inv + 64 * h * kTcLd + r;
       // (the inverse's 64 x 64 block of zeros is left out: an infinity in b stays on its side)
       if (h == (r >> 6) || (h == 0) == (p.lower_eff != 0)) {
@@ -200,19 +251,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
           for (int q = 0; q < NR; ++q) x[q] = fma(v, s.own[q * kTcBlock + 64 * h + k], x[q]);
         }
       }
-      if (h == 1) {
+    }
+    if (h == 1) {
 #pragma unroll
-        for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
-      }
-      __syncthreads();
-      if (h == 0) {
+      for (int q = 0; q < NR; ++q) s.part[q * kTcBlock + r] = x[q];
+    }
+    __syncthreads();
+    // A CTA that gave up leaves its rows as they are and sends NaN instead of x, so that the others'
+    // waits end; its own memory is written until their x is here (waited for below).
+    const bool late = s.late;
+    if (h == 0) {
 #pragma unroll
-        for (int q = 0; q < NR; ++q) {
-          const double v = r < nrow ? x[q] + s.part[q * kTcBlock + r] : 0.0;
-          s.own[q * kTcBlock + r] = v;
-          if (r < nrow && q < nr)
-            p.B[(int64_t)(r0 + r) * p.brs + (int64_t)(rhs0 + q) * p.bcs] = v;
-        }
+      for (int q = 0; q < NR; ++q) {
+        const double v = r < nrow ? x[q] + s.part[q * kTcBlock + r] : 0.0;
+        s.own[q * kTcBlock + r] = late ? __longlong_as_double(0x7ff8000000000000ll) : v;
+        if (r < nrow && q < nr && !late)
+          p.B[(int64_t)(r0 + r) * p.brs + (int64_t)(rhs0 + q) * p.bcs] = v;
       }
     }
     __syncthreads();
@@ -236,9 +290,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) trsm_cluster_kernel(const FewAr
   cl_sync();  // no CTA leaves while another may still write into its memory
 }
 
-template <typename TA, bool TRANS, int NR>
+template <typename TA, bool TRANS, int NR, bool UNIT>
 int tc_launch(mo_ctx *ctx, const FewArgs &p, int ctas, int groups) {
-  const void *fn = (const void *)trsm_cluster_kernel<TA, TRANS, NR>;
+  const void *fn = (const void *)trsm_cluster_kernel<TA, TRANS, NR, UNIT>;
   if (int rc = mo_smem_attr(fn, (int)sizeof(TcSmem<NR>))) return rc;
   MO_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
@@ -253,7 +307,7 @@ int tc_launch(mo_ctx *ctx, const FewArgs &p, int ctas, int groups) {
   cfg.numAttrs = 1;
   if (ctas > 8) {  // not portable: ask
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, trsm_cluster_kernel<TA, TRANS, NR>, &cfg) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveClusters(&clusters, trsm_cluster_kernel<TA, TRANS, NR, UNIT>, &cfg) != cudaSuccess ||
         clusters < 1) {
       cudaGetLastError();
       return 1;
@@ -279,13 +333,17 @@ int tc_run(mo_ctx *ctx, const FewArgs &p) {
   while (ctas < nblk) ctas *= 2;
   const int per = p.nrhs > 2 ? 4 : p.nrhs, groups = (p.nrhs + per - 1) / per;
   if (groups * ctas > 128) return 1;
-  if (p.trans)
-    return per == 1   ? tc_launch<TA, true, 1>(ctx, p, ctas, groups)
-           : per == 2 ? tc_launch<TA, true, 2>(ctx, p, ctas, groups)
-                      : tc_launch<TA, true, 4>(ctx, p, ctas, groups);
-  return per == 1   ? tc_launch<TA, false, 1>(ctx, p, ctas, groups)
-         : per == 2 ? tc_launch<TA, false, 2>(ctx, p, ctas, groups)
-                    : tc_launch<TA, false, 4>(ctx, p, ctas, groups);
+  auto go = [&](auto trans, auto unit) {
+    constexpr bool T = decltype(trans)::value, U = decltype(unit)::value;
+    return per == 1   ? tc_launch<TA, T, 1, U>(ctx, p, ctas, groups)
+           : per == 2 ? tc_launch<TA, T, 2, U>(ctx, p, ctas, groups)
+                      : tc_launch<TA, T, 4, U>(ctx, p, ctas, groups);
+  };
+  constexpr std::true_type yes{};
+  constexpr std::false_type no{};
+  if constexpr (sizeof(TA) == 8)  // (the mixed factor's triangles have no unit diagonal)
+    if (p.unit) return p.trans ? go(yes, yes) : go(no, yes);
+  return p.trans ? go(yes, no) : go(no, no);
 }
 
 }  // namespace

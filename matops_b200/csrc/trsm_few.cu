@@ -46,6 +46,7 @@ struct FewArgs {
   int64_t lda;
   bool trans;      // op(A) = A^T
   bool lower_eff;  // op(A) lower -> steps top-down
+  bool unit;       // unit diagonal (FP64 factors)
   int N, nblk;
   double *B;
   int64_t brs, bcs;  // element (i, c) of B at B[i*brs + c*bcs]
@@ -602,6 +603,7 @@ int few_run(mo_ctx *ctx, View B, const void *A, bool a32, int64_t lda, int N, in
   p.vec = ((uintptr_t)A % 16 == 0) && ((lda * (a32 ? 4 : 8)) % 16 == 0);
   p.trans = tr;
   p.lower_eff = lower_eff;
+  p.unit = !a32 && (flags & MO_UNIT) != 0;
   p.N = N;
   p.nblk = (N + TB - 1) / TB;
   p.B = B.d;
