@@ -76,6 +76,12 @@ struct CholSmem {
   double vec[MAXN];          // solve vector
   int idx, info;
 };
+// LARGE (orders above 128): with the running C of the tile that each tile warp has in hand, in
+// fragment order
+template <int T, bool LARGE>
+struct CholTiles : CholSmem {
+  double C[LARGE ? T / 32 * 3 / 4 : 1][LARGE ? CB * CB : 1];
+};
 
 static_assert(2 * LB * ULD <= (LB + 6) * (LB + 2), "two U12 tiles fit where L11 was");
 struct LuRow {
@@ -101,8 +107,10 @@ __device__ __forceinline__ double neg(double x) { return -x; }
 // acc (32 x 32: rows 16 mi + g + 8 h, columns 8 ni + 2 t + e at acc[mi][ni][2 h + e]) +=
 // sum over k of P(row, k) Q(column, k), K a multiple of 4, P and Q read from global memory in
 // fragment layout: `pa`, `pb` point at this lane's first element (row g, column g; k = t4).
+// fold() after every FOLD columns but the last ones.
+template <int FOLD, typename F>
 __device__ __forceinline__ void tile_mma(double (&acc)[2][4][4], const double *pa, const double *pb,
-                                         int64_t ld, int K) {
+                                         int64_t ld, int K, F &&fold) {
   double a[2][2][2], b[2][4];
   const int64_t step = 4 * ld;
   auto load = [&](int s) {
@@ -131,6 +139,7 @@ __device__ __forceinline__ void tile_mma(double (&acc)[2][4][4], const double *p
     mma(0);
     if (k + 8 < K) load(0);
     mma(1);
+    if ((k & (FOLD - 1)) == FOLD - 8 && k + 8 < K) fold();
   }
 }
 
@@ -286,35 +295,44 @@ __device__ __noinline__ void chol_diag(CholSmem &s, double *Ad, int64_t ld, int 
 // columns to their tiles of the next panel.  No tile warp shares warp 0's scheduler: beside
 // one warp of DMMAs a chain of FP64 FMAs is starved (512 of them take 200 K cycles instead
 // of 4.3 K; 1.5 M beside three).
-template <int T>
-__device__ int chol_matrix(CholSmem &s, double *A, int64_t ld, int n) {
+template <int T, bool LARGE>
+__device__ int chol_matrix(CholTiles<T, LARGE> &s, double *A, int64_t ld, int n) {
   constexpr int NT = T / 32 * 3 / 4;  // warps with panel tiles
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tw = warp % 4 ? warp - warp / 4 : 0;  // 1 .. NT: tile warps; 0: diagonal or idle
   const int g = lane >> 2, t4 = lane & 3;
   if (tid == 0) s.info = 0;
-  auto load_neg = [&](double (&acc)[2][4][4], int r0, int j) {
+  // f(index in fragment order, row and column in the tile, accumulator)
+  auto each = [&](double (&acc)[2][4][4], auto &&f) {
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int r = r0 + 16 * mi + g + 8 * (q >> 1), c = j + 8 * ni + 2 * t4 + (q & 1);
-          acc[mi][ni][q] = r < n && c < n && r >= c ? neg(A[r + (int64_t)c * ld]) : 0.0;
-        }
+        for (int q = 0; q < 4; ++q)
+          f(((mi * 4 + ni) * 4 + q) * 32 + lane, 16 * mi + g + 8 * (q >> 1),
+            8 * ni + 2 * t4 + (q & 1), acc[mi][ni][q]);
   };
-  // acc += L(rows r0.., k0 .. k0 + K) L(j .. j + 32, k0 .. k0 + K)^T
-  auto apply = [&](double (&acc)[2][4][4], int r0, int j, int k0, int K) {
+  // acc = L(rows r0.., 0 .. K) L(j .. j + 32, 0 .. K)^T, added up from zero.  LARGE: take(acc) takes the
+  // sum of every 32 columns but the last from the running C, so that C is rounded once per
+  // panel and shrinks from panel to panel, as in a right-looking factorization.  Error of L
+  // against one (geometric means), at diagonally dominant matrices of order 256 and 400, and
+  // at a condition of 1e6: with C in the accumulators, rounded by every product, 1.24 1.51,
+  // 1.55 1.93; all products from zero 0.75 0.76, 1.98 2.57; this way 0.73 0.76, 0.94 0.91.
+  // Times are the same as with C in the accumulators (512 x 256 0.29 ms, 600 x 512 3.1 -> 3.0); up to
+  // 128 columns the plain sum is 8 % faster and the difference small (order 128: 0.73, 1.38).
+  constexpr int kFold = LARGE ? CB : MAXN;
+  auto apply = [&](double (&acc)[2][4][4], int r0, int j, int K, auto &&take) {
     // (rows past n: the reads stay inside the matrix, since k < j < n and ld > 31 here, and
     // what they bring is not stored)
-    const double *base = A + g + (int64_t)(k0 + t4) * ld;
-    tile_mma(acc, base + r0, base + j, ld, K);
+    const double *base = A + g + (int64_t)t4 * ld;
+    each(acc, [](int, int, int, double &v) { v = 0.0; });
+    tile_mma<kFold>(acc, base + r0, base + j, ld, K, [&] {
+      take(acc);
+      each(acc, [](int, int, int, double &v) { v = 0.0; });
+    });
   };
-  // the diagonal tile's C, on its way to s.D while the products are added up from zero: with C
-  // in the accumulators every product was rounded to the last place of the large diagonal
-  // (error of L 2.9e-16 instead of 1.9e-16, of X 8.2e-16 instead of 6.2e-16 on diagonally dominant
-  // matrices of order 16 to 512; 2 % of the time)
+  // the diagonal tile's C, on its way to s.D meanwhile
   auto fetch_d = [&](int r0) {
 #pragma unroll 4
     for (int c = 0; c < CB; ++c) {
@@ -340,9 +358,27 @@ __device__ int chol_matrix(CholSmem &s, double *A, int64_t ld, int n) {
       double acc[2][4][4];
       const int r0 = j + t * CB;
       if (t < nt) {
-        // acc = -C, then += L L^T; the panel becomes -acc L11^-T
-        load_neg(acc, r0, j);
-        apply(acc, r0, j, 0, j);
+        // acc = L L^T - C; the panel becomes -acc L11^-T
+        double *At = A + r0 + (int64_t)j * ld;
+        auto in = [&](int r, int c) { return r0 + r < n && j + c < n && r0 + r >= j + c; };
+        const bool folds = LARGE && j > kFold;
+        double *C = s.C[LARGE ? tw - 1 : 0];
+        if (folds)
+          each(acc, [&](int e, int r, int c, double &) {
+            cp_async_8(C + e, in(r, c) ? At + r + (int64_t)c * ld : A, in(r, c) ? 8 : 0);
+          });
+        apply(acc, r0, j, j, [&](double (&d)[2][4][4]) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          each(d, [&](int e, int, int, double &v) { C[e] -= v; });
+        });
+        if (folds) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          each(acc, [&](int e, int, int, double &v) { v -= C[e]; });
+        } else {
+          each(acc, [&](int, int r, int c, double &v) {
+            if (in(r, c)) v -= At[r + (int64_t)c * ld];
+          });
+        }
       }
       if (!waited) {
         waited = true;
@@ -375,22 +411,13 @@ __device__ int chol_matrix(CholSmem &s, double *A, int64_t ld, int n) {
       if (t == 1) {  // the next diagonal tile: these rows, and the columns just stored too
         __syncwarp();
         fetch_d(r0);
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-        apply(acc, r0, r0, 0, r0);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              s.D[16 * mi + g + 8 * (q >> 1)][8 * ni + 2 * t4 + (q & 1)] -= acc[mi][ni][q];
+        auto take = [&](double (&d)[2][4][4]) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          __syncwarp();
+          each(d, [&](int, int r, int c, double &v) { s.D[r][c] -= v; });
+        };
+        apply(acc, r0, r0, r0, take);
+        take(acc);
       }
     }
   }
@@ -935,9 +962,10 @@ __device__ __noinline__ void solve_matrix(double *y, double (*D)[CB + 1], const 
   }
 }
 
-template <int T, int MINB>
+template <int T, int MINB, bool LARGE>
 __global__ void __launch_bounds__(T, MINB) batch_chol_kernel(BatchParams p) {
-  __shared__ CholSmem s;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto &s = *reinterpret_cast<CholTiles<T, LARGE> *>(smem_raw);
   for (;;) {
     if (threadIdx.x == 0) s.idx = atomicAdd(p.counter, 1);
     __syncthreads();
@@ -945,7 +973,7 @@ __global__ void __launch_bounds__(T, MINB) batch_chol_kernel(BatchParams p) {
     __syncthreads();
     if (q >= p.count) break;
     const int m = p.order[q], n = p.n[m];
-    const int info = chol_matrix<T>(s, p.A[m], p.lda[m], n);
+    const int info = chol_matrix<T, LARGE>(s, p.A[m], p.lda[m], n);
     if (threadIdx.x == 0) p.info[m] = info;
     if (p.B != nullptr && info == 0)
       solve_matrix<false, T>(s.vec, s.D, nullptr, p.A[m], p.lda[m], n, p.B[m], p.ldb[m], p.nrhs);
@@ -987,9 +1015,9 @@ struct KernelCfg {
   size_t smem;
 };
 
-template <int T, int MINB>
+template <int T, int MINB, bool LARGE>
 KernelCfg chol_cfg() {
-  return KernelCfg{T, (const void *)batch_chol_kernel<T, MINB>, 0};
+  return KernelCfg{T, (const void *)batch_chol_kernel<T, MINB, LARGE>, sizeof(CholTiles<T, LARGE>)};
 }
 template <int T, int RPT, int MINB>
 KernelCfg lu_cfg() {
@@ -1000,7 +1028,10 @@ KernelCfg lu_cfg() {
 // per SM; 1 = 128 threads, four CTAs per SM.  LU above 256 rows, where a thread holds at most
 // two rows: 0 = 512 threads, one CTA per SM, 1 = 256 threads, two CTAs per SM
 KernelCfg kernel_cfg(int kind, int b, int c) {
-  if (kind == MO_BATCH_CHOL) return c == 0 ? chol_cfg<256, 2>() : chol_cfg<128, 4>();
+  if (kind == MO_BATCH_CHOL) {
+    if (b >= NBUCKETS - 2) return c == 0 ? chol_cfg<256, 2, true>() : chol_cfg<128, 4, true>();
+    return c == 0 ? chol_cfg<256, 2, false>() : chol_cfg<128, 4, false>();
+  }
   if (b == NBUCKETS - 1) return c == 0 ? lu_cfg<512, 1, 1>() : lu_cfg<256, 2, 2>();
   if (c == 0) return lu_cfg<256, 1, 2>();
   return b == NBUCKETS - 2 ? lu_cfg<128, 2, 4>() : lu_cfg<128, 1, 4>();
