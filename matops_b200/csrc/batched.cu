@@ -33,8 +33,8 @@
 // few warps can do is kept short.  Measured on B200, 4096 systems n ~ U{16..512}, 1 RHS,
 // against right-looking 32-column panels with shared-memory staging (diagonal block, panel
 // substitution and solve by division chains; LU panels unrolled over 32 columns):
-// Cholesky 9.8 -> 5.75 ms, LU 40.3 -> 16.3; 512 x n = 256 Cholesky 0.94 -> 0.45 ms, LU 3.86 -> 1.46;
-// 1024 x n = 128 Cholesky 0.67 -> 0.22, LU 2.51 -> 0.64.
+// Cholesky 9.8 -> 5.8 ms, LU 42.7 -> 16.9; 512 x n = 256 Cholesky 0.60 -> 0.29 ms, LU 3.5 -> 1.3;
+// 1024 x n = 128 Cholesky 0.38 -> 0.13, LU 2.28 -> 0.57.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -1429,7 +1429,9 @@ extern "C" int mo_batch_create(mo_ctx *ctx, int kind, int count, const int32_t *
     b->bytes += 16.0 * ni * ni + 16.0 * ni * nrhs;
   }
   // default schedule (the autotuner may change it): more and smaller CTAs per SM, measured on
-  // 4096 systems of 16 to 512 unknowns: Cholesky 5.5 ms against 6.9, LU 16.5 against 19.1.
+  // 4096 systems of 16 to 512 unknowns: Cholesky 5.8 ms against 7.1, LU 16.9 against 19.8.
+  // (Only the order 257 to 512 of Cholesky, by 0: 200 x 512 1.05 ms against 1.27, 300 x 512 1.78
+  // against 1.47, the 4096 systems 6.9.)
   // LU from 129 to 256 rows: 256 threads (512 matrices of 256: 1.46 ms against 1.69)
   for (int &c : b->cfg) c = 1;
   if (kind == MO_BATCH_LU) b->cfg[2] = 0;

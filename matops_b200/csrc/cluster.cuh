@@ -1,5 +1,5 @@
 // Exchange between the CTAs of one thread-block cluster through distributed shared memory
-// (the LU and QR panels).
+// (the LU and QR panels; the triangular solves map addresses with it too).
 #pragma once
 #include "common.cuh"
 

@@ -6,10 +6,11 @@
 // first row holding the strict maximum of |x|; a NaN never wins unless it sits on the
 // diagonal, where the scan starts).  The factors do not depend on left- vs right-looking
 // order except through rounding, so the device runs the right-looking form:
-//   panel   : up to 16384 rows one thread-block cluster, rows in registers, one cluster
-//             barrier per column; above, a cooperative kernel whose CTAs own slices of the
-//             panel in shared memory, one grid barrier per column (candidate rows are
-//             published with the local argmax, so every CTA picks the pivot itself)
+//   panel   : up to 16384 rows one thread-block cluster, rows in registers, one exchange
+//             between the CTAs per column, through distributed shared memory onto an
+//             mbarrier; above, a cooperative kernel whose CTAs own slices of the panel in
+//             shared memory, one grid barrier per column (candidate rows are published with
+//             the local argmax, so every CTA picks the pivot itself)
 //   laswp   : apply the panel's interchanges to the other columns (all of them after the
 //             cluster panel, which leaves its rows where they were)
 //   trsm    : U12 = L11^-1 A12 (unit lower inverse + in-place GEMM)
@@ -250,9 +251,10 @@ __global__ void __launch_bounds__(PANEL_THREADS)
 // ---- the panel in one thread-block cluster ---------------------------------------------
 // What bounds a panel is its chain of columns: pivot search, exchange of the pivot row,
 // scaling, update, and nothing of column j + 1 can start before.  A grid barrier costs
-// several L2 round trips per column (5.0 us a column with the cooperative kernel below at
-// 1001 and at 16384 rows); inside a cluster the candidates travel through distributed shared
-// memory and one hardware barrier.  16 CTAs x 512 threads x 2 rows hold 16384 rows of a
+// several L2 round trips per column (5.0 us a column with the cooperative kernel above at
+// 1001 and at 16384 rows); inside a cluster the candidates and the diagonal row travel through
+// distributed shared memory onto one mbarrier per CTA and column (a cluster barrier comes
+// only between sub-panels).  16 CTAs x 256 threads x 4 rows hold 16384 rows of a
 // 16-column sub-panel in registers; the 128 columns are done left-looking, sub-panel by
 // sub-panel: a thread first applies the finished columns to its rows (L from L2, U from
 // shared memory), then the 16 columns are eliminated.  Every entry takes the same FMAs in
@@ -263,10 +265,11 @@ __global__ void __launch_bounds__(PANEL_THREADS)
 // matrix (the panel's among them) in order are emitted at the end.
 //
 // Measured on B200, 128 columns with the interchanges applied, against the cooperative
-// kernel: 128 rows 608 -> 187 us, 1001 rows 671 -> 256, 4000 rows 698 -> 264, 8000 rows 708 ->
+// kernel: 128 rows 608 -> 187 us, 1001 rows 671 -> 214, 4000 rows 698 -> 264, 8000 rows 708 ->
 // 320, 16000 rows 766 -> 439 (there the FP64 rate of the 16 SMs takes over).  A column takes
-// about 1000 cycles in one CTA and 1700 in a cluster, half of it the two argmax levels and
-// the exchange; the triangle of U and the left-looking products take the other third.
+// about 1000 cycles in one CTA and 1600 in a cluster, half of it the argmax and the exchange:
+// 65 us of the 187 and 104 of the 214.  The rest is the triangle of U by CTA 0 alone, its way
+// through global memory, and the left-looking products.
 constexpr int kClWarps = kClThreads / 32, kClSub = 16;
 constexpr int kClByWarp = 4, kClCands = kClByWarp * kClWarps;  // (one lane per candidate)
 constexpr int kClL = MAX_PANEL_W - kClSub;  // rows of U that a later sub-panel needs

@@ -799,8 +799,9 @@ int factor_block(mo_ctx *ctx, View A, int kb, int bo, int k, QrWork &q) {
 
 // The device part of DecomposeQRT / DecomposeQR: A (m x n) factored in place; T's upper
 // k x k triangle written when T.d, tau (k entries, stride tau_inc) when tau.  (Factoring
-// the next block on a second stream beside the trailing update was measured slower: the
-// update then runs without the panel's SMs and the T products without stream-K.)
+// the next block on a second stream beside the trailing update was slower with the
+// cooperative panel, which takes as many SMs as it has slices, and with the T products
+// without stream-K; with the cluster panel and its 16 SMs it has not been measured.)
 int qr_factor(mo_ctx *ctx, View A, View T, double *tau, int64_t tau_inc) {
   const int m = A.rows, n = A.cols, k = min(m, n);
   if (k == 0) return MO_OK;
