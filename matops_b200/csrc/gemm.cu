@@ -787,8 +787,11 @@ size_t gemm_partial_bytes(int sms) { return 2 * (size_t)sms * TILE_DBL * sizeof(
 // engine / small tiles in us: 64^3 12.3 / 4.1, 512 x 128 x 128 18.4 / 6.2, 1000 x 1000 x 128 24.6 /
 // 19.3, 500^3 32.8 / 18.4; above, 1500 x 1500 x 128 28.8 / 35.4, 800^3 51.2 / 61.6.  With A
 // transposed and B not, both operands' loads run across their columns, and past 1500 tiles the
-// small ones lose where there is more than one slab: 1414 x 1414 x 16 10.9 / 10.4, x 30 14.4 /
-// 16.5, x 68 20.6 / 26.7; 1000 x 1000 x 30, 1024 tiles, 12.5 / 10.3.
+// small ones lose where there is more than one slab and the engine's tiles fit C: 1414 x 1414 x
+// 16 10.9 / 10.4, x 30 14.4 / 16.5, x 68 20.6 / 26.7; 24000 x 128 x 30 16.5 / 20.6; but 160 x 10880 x
+// 30 26.8 / 12.7 and 96 x 32000 x 30 28.7 / 20.7 (tiles of 128 rows filled to 5/8 and 3/4), 54400
+// x 16 x 30 27.0 / 12.4; with more of K to hide the padding 200 x 8704 x 68 20.6 / 26.7.
+// 1000 x 1000 x 30, 1024 tiles, 12.5 / 10.3.
 // A C of a few small tiles with a long K is split along K, two CTAs per SM with at least 128
 // rows of K each, and the partial tiles are added in order by a second kernel: up to 2^29
 // multiply-adds, 128 x 128 x 8000 219 / 21, 512 x 128 x 8000 103 / 62, 1000 x 128 x 8000 101 / 119;
@@ -805,7 +808,12 @@ static int small_chunks(const GemmArgs &a, int sms) {
     const int chunks = (int)std::min<long long>(a.K / 128, 2 * sms / tiles);
     if (chunks > 1) return chunks;
   }
-  if (a.transA && !a.transB && a.C != a.B && tri * tiles > 1500 && a.K > BK) return 0;
+  if (a.transA && !a.transB && a.C != a.B && tri * tiles > 1500 && a.K > BK) {
+    auto up = [](double n, int t) { return std::ceil(n / t) * t; };
+    const bool wide = a.M <= 64 && a.N > 64;
+    const double padded = wide ? up(a.M, 64) * up(a.N, 128) : up(a.M, 128) * up(a.N, 64);
+    if (padded <= (a.K > 48 ? 1.4 : 1.25) * a.M * a.N) return 0;
+  }
   return a.K <= 4096 && work <= 134217728.0 ? 1 : 0;
 }
 
